@@ -1177,7 +1177,8 @@ int Engine::step(const EffRow * rows, size_t n_rows, OutRow * out_rows, int32_t 
     bool forced_outside_grammar = false;
     size_t top_stride = 0;
     bool any_v2 = false;       // some row needs the working copy of the logits
-    int n_greedy_fast = 0;
+    int n_greedy_fast = 0, n_chunked = 0;
+    bool sample_cands = false;      // some row is served from candidate lists
     {
         size_t s = 0;
         for (size_t r = 0; r < R; ++r) {
@@ -1268,6 +1269,11 @@ int Engine::step(const EffRow * rows, size_t n_rows, OutRow * out_rows, int32_t 
                 d.min_p = 0.f;
                 d.flags = 0;
             }
+            if (!(d.flags & 4u) && d.pad[0] == 0 && d.pad[1] == 0 && sample_chunked((int)hp.vocab, row.v2 != nullptr, d.top_k, d.min_p, d.top_p, d.n_top)) {
+                d.flags |= kSampleFlagChunked;
+                ++n_chunked;
+                sample_cands = sample_cands || d.n_top > 0 || (d.top_k > 0 && d.top_k < (int)hp.vocab);
+            }
         }
     }
 
@@ -1345,7 +1351,7 @@ int Engine::step(const EffRow * rows, size_t n_rows, OutRow * out_rows, int32_t 
         hs_.ensure(S * (size_t)hp.d);
         hs_split_.ensure(S, hp.d);
         if (any_v2) logits_work_.ensure(S * (size_t)hp.vocab);
-        if (n_greedy_fast) sample_scratch_.ensure(sample_scratch_bytes((int)hp.vocab, (int)S));
+        if (n_greedy_fast || n_chunked) sample_scratch_.ensure(sample_scratch_bytes((int)hp.vocab, (int)S, sample_cands));
     }
     if (any_adapter) {
         lora_tmp_.ensure((size_t)kLoraTcMaxTargets * kLoraTcMaxSplits * T * (size_t)std::max<uint32_t>(r_max_, 1));
@@ -1397,7 +1403,7 @@ int Engine::step(const EffRow * rows, size_t n_rows, OutRow * out_rows, int32_t 
     // eagerly, so every lazy allocation and kernel attribute is in place before a capture.
     last_h2d_bytes = stage_total;
     last_d2h_bytes = S ? res_total - 16 : 0;
-    const std::vector<uint64_t> sig = {R, T, S, (uint64_t)n_patches, (uint64_t)n_copies, edits.size(), top_stride, any_v2, (uint64_t)n_greedy_fast,
+    const std::vector<uint64_t> sig = {R, T, S, (uint64_t)n_patches, (uint64_t)n_copies, edits.size(), top_stride, any_v2, (uint64_t)n_greedy_fast, (uint64_t)n_chunked,
                                        any_adapter, (uint64_t)n_attn_items, (uint64_t)n_small_items, any_wide_item, any_mid_item,
                                        (uint64_t)attn_splits, stage_total, res_total, (uint64_t)result_bytes_, (uint64_t)adapters_.size(), (uint64_t)masks.size(),
                                        // a quantised pool's dequantisation grid covers the longest row's blocks
@@ -1596,14 +1602,11 @@ int Engine::step(const EffRow * rows, size_t n_rows, OutRow * out_rows, int32_t 
     if (S) {
         RB_K(K_OTHER, 1, launch_rms_norm(x_.ptr, d, maps.out_index, model->output_norm, d, hp.eps, hs_.ptr, d, (int)S, stream, hs_split_.get()));
         linear(model->output, hs_.ptr, d, (int)S, logits.ptr, (int)hp.vocab, model->output_bias, nullptr, 0, hs_split_.get());
-        if (any_v2) {
-            RB_CUDA(cudaMemcpyAsync(logits_work_.ptr, logits.ptr, S * (size_t)hp.vocab * 4, cudaMemcpyDeviceToDevice, stream));
-        }
-        RB_K(K_SAMPLE, (n_greedy_fast < (int)S ? 1 : 0) + (n_greedy_fast ? 2 : 0), launch_sample(logits.ptr, any_v2 ? logits_work_.ptr : nullptr, (int)hp.vocab, (int)S,
+        RB_K(K_SAMPLE, (n_greedy_fast + n_chunked ? 1 : 0) + (n_greedy_fast < (int)S ? 1 : 0) + (n_greedy_fast ? 1 : 0), launch_sample(logits.ptr, any_v2 ? logits_work_.ptr : nullptr, (int)hp.vocab, (int)S,
                                         reinterpret_cast<const SampleDesc *>(d_stage_.ptr + off_descs),
                                         reinterpret_cast<const LogitEdit *>(d_stage_.ptr + off_edits),
                                         masks.empty() ? nullptr : reinterpret_cast<const uint32_t *>(d_stage_.ptr + off_masks), d_out, d_top_ids, d_top_lps,
-                                        (int)std::max<size_t>(top_stride, 1), n_greedy_fast, sample_scratch_.ptr, stream));
+                                        (int)std::max<size_t>(top_stride, 1), n_greedy_fast, n_chunked, sample_scratch_.ptr, stream));
     }
 #undef RB_K
     if (S) RB_CUDA(cudaMemcpyAsync(h_result_, d_result_.ptr, res_total - 16, cudaMemcpyDeviceToHost, stream));

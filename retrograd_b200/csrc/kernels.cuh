@@ -183,6 +183,9 @@ struct RowDesc {
     int32_t pad1;
 };
 
+constexpr uint32_t kSampleFlagChunked = 8u;     // the row is finished from the chunks' statistics and candidates
+constexpr int kSampleMaxNeed = 128;             // largest top_k (or, without top_k, n_top) such a row may have
+
 // Per sampling row parameters (64 bytes).
 struct SampleDesc {
     float temperature;
@@ -193,7 +196,7 @@ struct SampleDesc {
     uint32_t draw_lo;     // per-request draw counter
     uint32_t draw_hi;
     uint32_t n_top;       // top logprobs requested
-    uint32_t flags;       // bit0: v2 row (post-transform reporting), bit1: want sampled_logprob, bit2: greedy without edits
+    uint32_t flags;       // bit0: v2 row (post-transform reporting), bit1: want sampled_logprob, bit2: greedy without edits, bit3: kSampleFlagChunked
     uint32_t edit_begin;  // range in the logit-edit list
     uint32_t edit_end;
     uint32_t pad[5];      // pad[0]: 1 + word offset of the row's grammar mask (0: none); pad[1]: 1 + the token a reasoning budget forces (0: none)
@@ -460,14 +463,19 @@ struct LoraGroup {
 void launch_lora_tc(const LoraGroup & group, const float * scales, int r_max, int n_in, int n_adapters, const int32_t * offsets, const int32_t * sorted,
                     const float * x, int ldx, int n_tokens, float * tmp, float * y, int ldy, cudaStream_t stream);
 
-// Sampling over logits rows [S][n_vocab]. v2 rows transform their row of `work_logits`, which must
-// then hold a copy of `raw_logits`; with v1 rows only, `work_logits` may be null.
-// Rows whose flags carry bit 2 (v2, top_k == 1, no logit edits) are served by chunked arg-max kernels
-// that need `scratch` (sample_scratch_bytes()); `n_greedy_fast` is how many rows carry the bit.
-size_t sample_scratch_bytes(int n_vocab, int n_rows);
+// Sampling over logits rows [S][n_vocab]. v2 rows of the general passes transform their row of `work_logits` (space
+// for S rows); with v1 rows only, `work_logits` may be null.
+// Rows whose flags carry bit 2 (v2, top_k == 1, no logit edits) or kSampleFlagChunked are served from per-chunk results
+// in `scratch` (sample_scratch_bytes(); `candidates`: some row asks for the largest values); `n_greedy_fast` is how
+// many rows carry bit 2.
+size_t sample_scratch_bytes(int n_vocab, int n_rows, bool candidates);
+// Whether a row with these options is served from per-chunk results (the caller then sets kSampleFlagChunked, provided the row
+// has no grammar mask and no forced token).
+bool sample_chunked(int n_vocab, bool v2, int top_k, float min_p, float top_p, uint32_t n_top);
 // `masks`: grammar rows carry in desc.pad[0] the word offset (plus one) of their one-bit-per-token mask; null without such rows.
+// `n_chunked`: rows that carry kSampleFlagChunked.
 void launch_sample(const float * raw_logits, float * work_logits, int n_vocab, int n_rows, const SampleDesc * desc, const LogitEdit * edits,
-                   const uint32_t * masks, SampleOut * out, int32_t * top_ids, float * top_logprobs, int top_stride, int n_greedy_fast, void * scratch,
-                   cudaStream_t stream);
+                   const uint32_t * masks, SampleOut * out, int32_t * top_ids, float * top_logprobs, int top_stride, int n_greedy_fast, int n_chunked,
+                   void * scratch, cudaStream_t stream);
 
 } // namespace rb200

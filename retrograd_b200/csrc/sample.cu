@@ -1,4 +1,11 @@
-// On-device sampling for the step's output rows: one 1024-thread block per logits row.
+// On-device sampling for the step's output rows.
+//
+// A row of 128 256 logits read a dozen times by one block took 2.1 ms for 30 rows and 5.6 ms for 320 (top_k 20): the
+// passes were serial, and most of them only looked for values that top_k had removed long before. Rows are now cut
+// into chunks of 4096 logits that separate blocks read ONCE (sample_chunk_kernel: maximum, sum of exponentials, and the
+// chunk's candidates for the largest `need` values), and one block per row finishes from the chunks' results
+// (sample_kernel, row_from_chunks). The general passes remain for rows the chunks cannot serve: grammar masks, forced
+// tokens, a nucleus over the whole vocabulary, top_k above kMaxNeed, and rows whose ties overflow a candidate list.
 //
 // What is reproduced from the reference's CPU oracle
 // (crates/retrograd-ffi/runtime/src/retro_gen_core.cpp:41-51,103-225,718-875,2942-2985):
@@ -23,7 +30,30 @@ namespace rb200 {
 namespace {
 
 constexpr int kThreads = 1024;
-constexpr uint32_t kFlagV2 = 1u, kFlagWantLogprob = 2u, kFlagGreedyFast = 4u;
+constexpr uint32_t kFlagV2 = 1u, kFlagWantLogprob = 2u, kFlagGreedyFast = 4u, kFlagChunked = kSampleFlagChunked;
+
+constexpr int kChunk = 4096, kChunkThreads = 256;
+constexpr int kMaxNeed = kSampleMaxNeed;        // largest top_k / n_top served from candidate lists
+constexpr int kChunkCands = 256;                // candidates a chunk may hand on: about 174 of 4096 random values for need = 128
+constexpr int kRowCands = 4096;                 // candidates of a row the finishing block stages in shared memory
+constexpr int kListMax = 256;                   // values at or above the row's need-th largest (ties included)
+
+struct ChunkStat {
+    double sum;      // sum of exp(l - max) over the chunk's raw logits, fixed order
+    double tsum;     // sum of exp((e - emax) / T) over its edited logits; only for rows without top_k
+    float max;
+    int32_t arg;     // lowest id holding the maximum
+    float emax;      // maximum of the edited logits
+    int32_t earg;
+    int32_t count;   // candidates found (more than kChunkCands: the list is incomplete)
+    int32_t pad[3];
+};
+static_assert(sizeof(ChunkStat) == 48, "ChunkStat layout");
+
+struct Cand {
+    float v;
+    int32_t id;
+};
 
 struct Shared {
     double dwarp[32];
@@ -206,19 +236,466 @@ __device__ void radix_select(Shared & sh, const float * __restrict__ l, int V, b
     *above = acc_above;
 }
 
+__device__ __forceinline__ float edited(float v, const LogitEdit & ed) {
+    float t = v + ed.bias;
+    if (ed.repeat != 1.0f) t = t <= 0.0f ? t * ed.repeat : t / ed.repeat;
+    return t - ed.subtract;
+}
+
+// Rows of the chunked paths by their options: the values that matter are the edited ones for v2 rows.
+__device__ __forceinline__ bool truncates(const SampleDesc & d, int V) { return (d.flags & kFlagV2) && d.top_k > 0 && d.top_k < V; }
+__device__ __forceinline__ int needed(const SampleDesc & d, int V, int top_stride) {
+    return truncates(d, V) ? d.top_k : (int)min(d.n_top, (uint32_t)min(top_stride, V));
+}
+
+// One chunk of one row, read once into registers (16 values per thread). Bound by the double-precision exponentials
+// of the log-sum (one per logit), not by memory: 257 rows of 201 088 logits take 130 us, 1.6 TB/s.
+// Candidates: with `need` values wanted of the whole row, the need-th largest of the 256 per-thread maxima is a lower
+// bound of the chunk's need-th largest value; everything at or above it goes to the list (a few more than `need`).
+__global__ void __launch_bounds__(kChunkThreads) sample_chunk_kernel(const float * __restrict__ raw_logits, int V, const SampleDesc * __restrict__ descs,
+                                                                     const LogitEdit * __restrict__ edits, ChunkStat * __restrict__ stats,
+                                                                     Cand * __restrict__ cands, int n_chunks, int top_stride) {
+    const int row = blockIdx.y, chunk = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const SampleDesc d = descs[row];
+    if (!(d.flags & (kFlagGreedyFast | kFlagChunked))) return;
+    constexpr int PER = kChunk / kChunkThreads;
+    __shared__ float s_max[kChunkThreads / 32];
+    __shared__ int32_t s_arg[kChunkThreads / 32];
+    __shared__ double s_sum[kChunkThreads / 32];
+    __shared__ float s_val[kChunk];
+    __shared__ int s_count;
+    const float * l = raw_logits + (size_t)row * V;
+    const int base = chunk * kChunk;
+    float v[PER];
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const int i = base + j * kChunkThreads + tid;
+        v[j] = i < V ? l[i] : -INFINITY;
+    }
+    auto block_max = [&](float & m, int32_t & a) {
+        m = -INFINITY;
+        a = 0x7fffffff;
+#pragma unroll
+        for (int j = 0; j < PER; ++j)
+            if (v[j] > m) { m = v[j]; a = base + j * kChunkThreads + tid; }       // ascending ids: the first maximum wins
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float om = __shfl_xor_sync(0xffffffffu, m, o);
+            const int32_t oa = __shfl_xor_sync(0xffffffffu, a, o);
+            if (om > m || (om == m && oa < a)) { m = om; a = oa; }
+        }
+        __syncthreads();
+        if (lane == 0) { s_max[wid] = m; s_arg[wid] = a; }
+        __syncthreads();
+        m = s_max[0];
+        a = s_arg[0];
+#pragma unroll
+        for (int w = 1; w < kChunkThreads / 32; ++w)
+            if (s_max[w] > m || (s_max[w] == m && s_arg[w] < a)) { m = s_max[w]; a = s_arg[w]; }
+    };
+    auto block_exp_sum = [&](float m, double inv_t) {       // the sum, in thread 0
+        double part = 0.0;
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            const int i = base + j * kChunkThreads + tid;
+            if (i < V) part += exp(((double)v[j] - (double)m) * inv_t);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+        __syncthreads();
+        if (lane == 0) s_sum[wid] = part;
+        __syncthreads();
+        double sum = 0.0;
+        if (tid == 0) {
+#pragma unroll
+            for (int w = 0; w < kChunkThreads / 32; ++w) sum += s_sum[w];
+        }
+        return sum;
+    };
+    ChunkStat st;
+    block_max(st.max, st.arg);
+    st.sum = block_exp_sum(st.max, 1.0);
+    st.emax = st.max;
+    st.earg = st.arg;
+    st.tsum = st.sum;
+    st.count = 0;
+    st.pad[0] = st.pad[1] = st.pad[2] = 0;
+    if (d.flags & kFlagChunked) {
+        const uint32_t n_edits = (d.flags & kFlagV2) ? d.edit_end - d.edit_begin : 0u;
+        if (n_edits) {
+#pragma unroll
+            for (int j = 0; j < PER; ++j) s_val[j * kChunkThreads + tid] = v[j];
+            __syncthreads();
+            for (uint32_t e = tid; e < n_edits; e += kChunkThreads) {       // one edit per distinct id
+                const LogitEdit ed = edits[d.edit_begin + e];
+                const int at = ed.id - base;
+                if (at >= 0 && at < kChunk && ed.id < V) s_val[at] = edited(s_val[at], ed);
+            }
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < PER; ++j) v[j] = s_val[j * kChunkThreads + tid];
+            block_max(st.emax, st.earg);
+        }
+        const double inv_t = 1.0 / (double)d.temperature;
+        if (!truncates(d, V) && (n_edits || inv_t != 1.0)) st.tsum = block_exp_sum(st.emax, inv_t);
+        const int need = needed(d, V, top_stride);
+        if (need > 0) {
+            uint32_t mine = 0;
+#pragma unroll
+            for (int j = 0; j < PER; ++j) mine = max(mine, order_key(v[j]));
+            uint32_t bound = 0;        // the need-th largest of the threads' maxima, bit by bit
+            for (int bit = 31; bit >= 0; --bit) {
+                const uint32_t t = bound | (1u << bit);
+                if (__syncthreads_count(mine >= t) >= need) bound = t;
+            }
+            if (tid == 0) s_count = 0;
+            __syncthreads();
+            Cand * list = cands + ((size_t)row * n_chunks + chunk) * kChunkCands;
+#pragma unroll
+            for (int j = 0; j < PER; ++j) {
+                const int i = base + j * kChunkThreads + tid;
+                if (i < V && order_key(v[j]) >= bound) {
+                    const int at = atomicAdd(&s_count, 1);       // (the order in the list does not matter)
+                    if (at < kChunkCands) list[at] = Cand{v[j], i};
+                }
+            }
+            __syncthreads();
+            st.count = s_count;
+        }
+    }
+    if (tid == 0) stats[(size_t)row * n_chunks + chunk] = st;
+}
+
+// What row_from_chunks works with besides Shared.
+struct RowShared {
+    float cv[kRowCands];            // the row's candidates; later the drawn chunk's edited logits
+    int32_t cid[kRowCands];
+    float sv[kListMax];             // the kept values, largest first (ties: lowest id first)
+    int32_t sid[kListMax];
+    double p[kListMax];
+    float lv[kListMax];             // the list before it is ordered
+    int32_t lid[kListMax];
+    int32_t by_id[kListMax];        // kept entries in id order
+    int32_t offset[kThreads];       // first candidate of each chunk
+    double total, rtotal, mass, prefix;
+    float rmax, tmax;
+    int32_t rarg, targ, n_keep, token, chunk, n_list;
+};
+
+// The last step of a row whose chunks hold everything it needs; false when they do not (more ties than the lists take):
+// the caller then runs the general passes. Follows the general kernel's rules line by line (the comments there).
+__device__ bool row_from_chunks(Shared & sh, RowShared & rs, const float * __restrict__ raw, int V, const SampleDesc & d, const LogitEdit * __restrict__ edits,
+                                const ChunkStat * __restrict__ st, const Cand * __restrict__ cands, int n_chunks, SampleOut * __restrict__ out,
+                                int32_t * __restrict__ top_ids, float * __restrict__ top_lps, int top_stride) {
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const bool v2 = (d.flags & kFlagV2) != 0, cut = truncates(d, V);
+    const int need = needed(d, V, top_stride);
+    const double inv_t = 1.0 / (double)d.temperature;
+    // ---- the row's statistics from its chunks'
+    if (wid == 0) {
+        float m = -INFINITY, em = -INFINITY;
+        int32_t a = 0x7fffffff, ea = 0x7fffffff;
+        for (int c = lane; c < n_chunks; c += 32) {
+            if (st[c].max > m || (st[c].max == m && st[c].arg < a)) { m = st[c].max; a = st[c].arg; }
+            if (st[c].emax > em || (st[c].emax == em && st[c].earg < ea)) { em = st[c].emax; ea = st[c].earg; }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float om = __shfl_xor_sync(0xffffffffu, m, o), oem = __shfl_xor_sync(0xffffffffu, em, o);
+            const int32_t oa = __shfl_xor_sync(0xffffffffu, a, o), oea = __shfl_xor_sync(0xffffffffu, ea, o);
+            if (om > m || (om == m && oa < a)) { m = om; a = oa; }
+            if (oem > em || (oem == em && oea < ea)) { em = oem; ea = oea; }
+        }
+        double total = 0.0, ttotal = 0.0;
+        for (int c = lane; c < n_chunks; c += 32) {
+            total += st[c].sum * exp((double)st[c].max - (double)m);
+            if (!cut) ttotal += st[c].tsum * exp(((double)st[c].emax - (double)em) * inv_t);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            total += __shfl_xor_sync(0xffffffffu, total, o);
+            ttotal += __shfl_xor_sync(0xffffffffu, ttotal, o);
+        }
+        if (lane == 0) { rs.rmax = m; rs.rarg = a; rs.tmax = em; rs.targ = ea; rs.rtotal = total; rs.total = ttotal; }
+    }
+    // ---- the largest `need` values, exactly
+    int n_list = 0;
+    if (need > 0) {
+        int32_t n_cand;
+        int32_t mine = 0;
+        bool over = false;
+        if (tid < n_chunks) { mine = st[tid].count; over = mine > kChunkCands; }
+        const int32_t first = block_exclusive_scan_int(sh, mine, &n_cand);
+        rs.offset[tid] = first;
+        if (__syncthreads_or(over) || n_cand > kRowCands) return false;
+        for (int c = wid; c < n_chunks; c += kThreads / 32) {
+            const int n = st[c].count, at = rs.offset[c];
+            for (int i = lane; i < n; i += 32) {
+                const Cand e = cands[(size_t)c * kChunkCands + i];
+                rs.cv[at + i] = e.v;
+                rs.cid[at + i] = e.id;
+            }
+        }
+        __syncthreads();
+        uint32_t key[kRowCands / kThreads];
+        const int slots = (n_cand + kThreads - 1) / kThreads;
+#pragma unroll
+        for (int m = 0; m < kRowCands / kThreads; ++m) {
+            const int i = m * kThreads + tid;
+            key[m] = i < n_cand ? order_key(rs.cv[i]) : 0u;        // (no float has key 0)
+        }
+        auto count_from = [&](uint32_t t) {
+            int n = 0;
+#pragma unroll
+            for (int m = 0; m < kRowCands / kThreads; ++m)
+                if (m < slots) n += __syncthreads_count(key[m] >= t);
+            return n;
+        };
+        uint32_t thr = 0;
+        if (n_cand > need) {
+            for (int bit = 31; bit >= 0; --bit) {
+                const uint32_t t = thr | (1u << bit);
+                if (count_from(t) >= need) thr = t;
+            }
+        }
+        thr = max(thr, 1u);
+        n_list = count_from(thr);
+        if (n_list > kListMax) return false;
+        if (tid == 0) rs.n_list = 0;
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; m < kRowCands / kThreads; ++m) {
+            if (m < slots && key[m] >= thr) {
+                const int at = atomicAdd(&rs.n_list, 1);
+                rs.lv[at] = rs.cv[m * kThreads + tid];
+                rs.lid[at] = rs.cid[m * kThreads + tid];
+            }
+        }
+        __syncthreads();
+        if (tid < n_list) {
+            const float v = rs.lv[tid];
+            const int32_t id = rs.lid[tid];
+            int rank = 0;
+            for (int i = 0; i < n_list; ++i) rank += rs.lv[i] > v || (rs.lv[i] == v && rs.lid[i] < id);
+            rs.sv[rank] = v;
+            rs.sid[rank] = id;
+        }
+        n_list = min(n_list, need);        // ties beyond the need-th value: the lowest ids stay
+    }
+    __syncthreads();
+    const float rmax = rs.rmax;
+    const double rlog = log(rs.rtotal);
+    float tmax = rs.tmax;
+    int32_t token;
+    double kept;
+    bool single;
+    int n_keep = n_list;
+    if (cut) {
+        // ---- top_k, min_p, temperature and top_p on the kept list
+        tmax = rs.sv[0];
+        if (d.min_p > 0.0f) {
+            const float thr = tmax + logf(d.min_p);
+            n_keep = __syncthreads_count(tid < n_list && rs.sv[min(tid, kListMax - 1)] >= thr);
+        }
+        if (tid < n_keep) rs.p[tid] = exp(((double)rs.sv[tid] - (double)tmax) * inv_t);
+        __syncthreads();
+        const double total = block_sum(sh, tid < n_keep ? rs.p[tid] : 0.0);
+        single = d.top_k == 1 || (double)d.top_p * total <= 1.0;
+        if (!single && d.top_p < 1.0f) {
+            const unsigned long long w = tid < n_keep ? (unsigned long long)(rs.p[tid] * 1099511627776.0) : 0ull;
+            const double total_fixed = block_sum(sh, (double)w);
+            unsigned long long target = (unsigned long long)((double)d.top_p * total_fixed);
+            if (target < 1ull) target = 1ull;
+            if (tid == 0) {
+                unsigned long long above = 0;
+                int keep = n_keep;
+                for (int i = 0; i < n_keep;) {
+                    int j = i + 1;
+                    while (j < n_keep && rs.sv[j] == rs.sv[i]) ++j;
+                    const unsigned long long one = (unsigned long long)(rs.p[i] * 1099511627776.0);
+                    if (above + one * (unsigned long long)(j - i) >= target) {
+                        const unsigned long long lack = target > above ? target - above : 1ull;
+                        const unsigned long long ties = one ? (lack + one - 1) / one : 1ull;
+                        keep = i + (int)min((unsigned long long)(j - i), max(ties, 1ull));
+                        break;
+                    }
+                    above += one * (unsigned long long)(j - i);
+                    i = j;
+                }
+                rs.n_keep = keep;
+            }
+            __syncthreads();
+            n_keep = rs.n_keep;
+        }
+        if (single) {
+            token = rs.sid[0];
+            kept = 1.0;
+        } else {
+            if (tid < n_keep) {
+                const int32_t id = rs.sid[tid];
+                int rank = 0;
+                for (int i = 0; i < n_keep; ++i) rank += rs.sid[i] < id;
+                rs.by_id[rank] = tid;
+            }
+            __syncthreads();
+            if (tid == 0) {
+                double mass = 0.0;
+                for (int i = 0; i < n_keep; ++i) mass += rs.p[rs.by_id[i]];
+                const double draw = philox_uniform(d.seed, d.draw_lo, d.draw_hi) * mass;
+                double acc = 0.0;
+                int32_t pick = -1;
+                for (int i = 0; i < n_keep; ++i) {
+                    const double p = rs.p[rs.by_id[i]];
+                    if (p <= 0.0) continue;
+                    acc += p;
+                    pick = rs.sid[rs.by_id[i]];
+                    if (draw < acc) break;
+                }
+                rs.mass = mass;
+                rs.token = pick;
+            }
+            __syncthreads();
+            token = rs.token;
+            kept = rs.mass;
+        }
+    } else {
+        // ---- no truncation: the chunk the draw falls into, then the token within it
+        single = (double)d.top_p * rs.total <= 1.0;
+        kept = single ? 1.0 : rs.total;
+        token = rs.targ;
+        if (!single) {
+            if (tid == 0) {
+                const double draw = philox_uniform(d.seed, d.draw_lo, d.draw_hi) * rs.total;
+                double acc = 0.0;
+                int pick = -1;
+                double before = 0.0;
+                for (int c = 0; c < n_chunks; ++c) {
+                    const double mass = st[c].tsum * exp(((double)st[c].emax - (double)tmax) * inv_t);
+                    if (!(mass > 0.0)) continue;
+                    pick = c;
+                    before = acc;
+                    acc += mass;
+                    if (draw < acc) break;
+                }
+                rs.chunk = max(pick, 0);
+                rs.prefix = before;
+                rs.mass = draw;
+                rs.token = -1;
+            }
+            __syncthreads();
+            const int base = rs.chunk * kChunk;
+            for (int i = tid; i < kChunk; i += kThreads) rs.cv[i] = base + i < V ? raw[base + i] : -INFINITY;
+            __syncthreads();
+            if (v2) {
+                for (uint32_t e = d.edit_begin + tid; e < d.edit_end; e += kThreads) {
+                    const LogitEdit ed = edits[e];
+                    const int at = ed.id - base;
+                    if (at >= 0 && at < kChunk && ed.id < V) rs.cv[at] = edited(rs.cv[at], ed);
+                }
+            }
+            __syncthreads();
+            constexpr int PER = kChunk / kThreads;
+            double p[PER], mine = 0.0;
+            int32_t my_last = -1;
+#pragma unroll
+            for (int j = 0; j < PER; ++j) {
+                p[j] = base + tid * PER + j < V ? exp(((double)rs.cv[tid * PER + j] - (double)tmax) * inv_t) : 0.0;
+                if (p[j] > 0.0) { mine += p[j]; my_last = base + tid * PER + j; }
+            }
+            const double before = rs.prefix + block_exclusive_scan(sh, mine, nullptr);
+            const double draw = rs.mass;
+            if (mine > 0.0 && draw >= before && draw < before + mine) {
+                double acc = before;
+                int32_t pick = -1;
+#pragma unroll
+                for (int j = 0; j < PER; ++j) {
+                    acc += p[j];
+                    if (pick < 0 && p[j] > 0.0 && draw < acc) pick = base + tid * PER + j;
+                }
+                rs.token = pick < 0 ? my_last : pick;
+            }
+            __syncthreads();
+            if (rs.token < 0) {
+                // rounding left the draw past the last boundary (or between two threads' sums): the chunk's last token
+                float dummy;
+                int32_t last;
+                block_argmax(sh, (float)my_last, -my_last, dummy, last);
+                token = (int32_t)dummy;
+            } else {
+                token = rs.token;
+            }
+        }
+    }
+    // ---- outputs
+    const uint32_t n_top = min(d.n_top, (uint32_t)min(top_stride, V));
+    if (n_top > 0 && !v2) {
+        if ((uint32_t)tid < n_top) {
+            top_ids[tid] = rs.sid[tid];
+            top_lps[tid] = (float)((double)rs.sv[tid] - (double)rmax - rlog);
+        }
+    } else if (n_top > 0) {
+        const uint32_t shown = single ? 1u : min(n_top, (uint32_t)n_keep);
+        if ((uint32_t)tid < shown) {
+            top_ids[tid] = single ? token : rs.sid[tid];
+            top_lps[tid] = (float)log(exp(((double)(single ? tmax : rs.sv[tid]) - (double)tmax) * inv_t) / kept);
+        }
+        if (tid == 0) {
+            // everything else was truncated away: ids in ascending order, probability zero
+            int32_t id = 0;
+            for (uint32_t j = shown; j < n_top; ++j, ++id) {
+                for (bool taken = true; taken;) {
+                    taken = false;
+                    for (uint32_t i = 0; i < shown; ++i) taken = taken || (single ? token : rs.sid[i]) == id;
+                    if (taken) ++id;
+                }
+                top_ids[j] = id;
+                top_lps[j] = (float)log(exp(-INFINITY * inv_t) / kept);
+            }
+        }
+    }
+    if (token < 0 || token >= V) token = 0;      // a row of NaNs has no arg-max: stay inside the row
+    if (tid == 0) {
+        SampleOut o;
+        o.token = token;
+        o.logprob = (float)((double)raw[token] - (double)rmax - rlog);
+        o.sampled_logprob = 0.f;
+        if (v2 && (d.flags & kFlagWantLogprob)) {
+            float lt = raw[token];
+            for (uint32_t e = d.edit_begin; e < d.edit_end; ++e)
+                if (edits[e].id == token) lt = edited(lt, edits[e]);
+            o.sampled_logprob = (float)log(exp(((double)lt - (double)tmax) * inv_t) / kept);
+        }
+        o.n_top = n_top;
+        *out = o;
+    }
+    return true;
+}
+
 __global__ void __launch_bounds__(kThreads) sample_kernel(const float * __restrict__ raw_logits, float * __restrict__ work_logits, int V,
                                                           const SampleDesc * __restrict__ descs, const LogitEdit * __restrict__ edits,
-                                                          const uint32_t * __restrict__ masks, SampleOut * __restrict__ outs,
+                                                          const uint32_t * __restrict__ masks, const ChunkStat * __restrict__ stats,
+                                                          const Cand * __restrict__ cands, int n_chunks, SampleOut * __restrict__ outs,
                                                           int32_t * __restrict__ top_ids, float * __restrict__ top_lps, int top_stride) {
     __shared__ Shared sh;
+    extern __shared__ __align__(16) unsigned char row_shared[];
     const int row = blockIdx.x;
     const SampleDesc d = descs[row];
-    if (d.flags & kFlagGreedyFast) return;      // served by the chunked arg-max kernels below
+    if (d.flags & kFlagGreedyFast) return;      // served by greedy_finish_kernel
     const bool v2 = (d.flags & kFlagV2) != 0;
-    // v2 rows transform a private copy of their row; v1 rows only read the raw one
     const float * raw = raw_logits + (size_t)row * V;
-    float * l = v2 ? work_logits + (size_t)row * V : const_cast<float *>(raw);
     const int tid = threadIdx.x;
+    if ((d.flags & kFlagChunked) &&
+        row_from_chunks(sh, *reinterpret_cast<RowShared *>(row_shared), raw, V, d, edits, stats + (size_t)row * n_chunks,
+                        cands + (size_t)row * n_chunks * kChunkCands, n_chunks, outs + row, top_ids + (size_t)row * top_stride,
+                        top_lps + (size_t)row * top_stride, top_stride))
+        return;
+    // ---- the general passes: v2 rows transform a private copy of their row; v1 rows only read the raw one
+    float * l = v2 ? work_logits + (size_t)row * V : const_cast<float *>(raw);
+    __syncthreads();
+    if (v2) {
+        for (int i = tid; i < V; i += kThreads) l[i] = raw[i];        // (every pass below reads a thread's own elements or follows a barrier)
+        __syncthreads();
+    }
 
     // ---- temperature-1 statistics of the raw row
     float rmax = -INFINITY;
@@ -262,10 +739,7 @@ __global__ void __launch_bounds__(kThreads) sample_kernel(const float * __restri
         // logit_bias and penalties: one merged edit per distinct id
         for (uint32_t e = tid; e < n_edits; e += kThreads) {
             const LogitEdit ed = edits[d.edit_begin + e];
-            float t = l[ed.id] + ed.bias;
-            if (ed.repeat != 1.0f) t = t <= 0.0f ? t * ed.repeat : t / ed.repeat;
-            t -= ed.subtract;
-            l[ed.id] = t;
+            l[ed.id] = edited(l[ed.id], ed);
         }
         __syncthreads();
         // grammar mask: one bit per token, tokens the grammar cannot continue with drop out here
@@ -466,85 +940,32 @@ __global__ void __launch_bounds__(kThreads) sample_kernel(const float * __restri
 }
 
 
-// ---- greedy rows without logit edits (v2, top_k == 1): the token is the arg-max of the raw row and
-// the only statistics needed are the row's maximum and its double-precision sum of exponentials.
-// The row is cut into chunks of kChunk logits handled by separate blocks, so a handful of rows still
-// fills the GPU; a second tiny kernel merges the chunk results in chunk order.
-constexpr int kChunk = 4096, kChunkThreads = 256;
-
-struct ChunkStat {
-    double sum;      // sum of exp(l - max) over the chunk, fixed order
-    float max;
-    int32_t arg;     // lowest id holding the maximum
-};
-static_assert(sizeof(ChunkStat) == 16, "ChunkStat layout");
-
-__global__ void __launch_bounds__(kChunkThreads) greedy_chunk_kernel(const float * __restrict__ raw_logits, int V, const SampleDesc * __restrict__ descs,
-                                                                     ChunkStat * __restrict__ stats, int n_chunks) {
-    const int row = blockIdx.y, chunk = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    if (!(descs[row].flags & kFlagGreedyFast)) return;
-    __shared__ float s_max[kChunkThreads / 32];
-    __shared__ int32_t s_arg[kChunkThreads / 32];
-    __shared__ double s_sum[kChunkThreads / 32];
-    const float * l = raw_logits + (size_t)row * V;
-    const int base = chunk * kChunk;
-    float v[kChunk / kChunkThreads];
-    float m = -INFINITY;
-    int32_t a = 0x7fffffff;
-#pragma unroll
-    for (int j = 0; j < kChunk / kChunkThreads; ++j) {
-        const int i = base + j * kChunkThreads + tid;
-        v[j] = i < V ? l[i] : -INFINITY;
-        if (v[j] > m) { m = v[j]; a = i; }       // ascending ids: the first maximum wins
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float om = __shfl_xor_sync(0xffffffffu, m, o);
-        const int32_t oa = __shfl_xor_sync(0xffffffffu, a, o);
-        if (om > m || (om == m && oa < a)) { m = om; a = oa; }
-    }
-    if (lane == 0) { s_max[wid] = m; s_arg[wid] = a; }
-    __syncthreads();
-    m = s_max[0];
-    a = s_arg[0];
-#pragma unroll
-    for (int w = 1; w < kChunkThreads / 32; ++w)
-        if (s_max[w] > m || (s_max[w] == m && s_arg[w] < a)) { m = s_max[w]; a = s_arg[w]; }
-    double part = 0.0;
-#pragma unroll
-    for (int j = 0; j < kChunk / kChunkThreads; ++j) {
-        const int i = base + j * kChunkThreads + tid;
-        if (i < V) part += exp((double)v[j] - (double)m);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    if (lane == 0) s_sum[wid] = part;
-    __syncthreads();
-    if (tid == 0) {
-        double sum = 0.0;
-#pragma unroll
-        for (int w = 0; w < kChunkThreads / 32; ++w) sum += s_sum[w];
-        ChunkStat st;
-        st.sum = sum;
-        st.max = m;
-        st.arg = a;
-        stats[(size_t)row * n_chunks + chunk] = st;
-    }
-}
-
+// ---- greedy rows without logit edits (v2, top_k == 1): the token is the arg-max of the raw row and the only statistics
+// needed are the row's maximum and its double-precision sum of exponentials. One warp per row merges the chunks'
+// results (a single thread walking 32 chunks took 8.7 us, a dependent chain of loads and exponentials).
 __global__ void greedy_finish_kernel(const float * __restrict__ raw_logits, int V, const SampleDesc * __restrict__ descs,
                                      const ChunkStat * __restrict__ stats, int n_chunks, SampleOut * __restrict__ outs,
                                      int32_t * __restrict__ top_ids, float * __restrict__ top_lps, int top_stride) {
     const int row = blockIdx.x;
     const SampleDesc d = descs[row];
-    if (!(d.flags & kFlagGreedyFast) || threadIdx.x != 0) return;
+    if (!(d.flags & kFlagGreedyFast)) return;
     const ChunkStat * st = stats + (size_t)row * n_chunks;
-    float rmax = st[0].max;
-    int32_t token = st[0].arg;
-    for (int c = 1; c < n_chunks; ++c)
-        if (st[c].max > rmax) { rmax = st[c].max; token = st[c].arg; }      // chunks ascend in id: strict > keeps the lowest id
+    const int lane = threadIdx.x;
+    float rmax = -INFINITY;
+    int32_t token = 0x7fffffff;
+    for (int c = lane; c < n_chunks; c += 32)
+        if (st[c].max > rmax || (st[c].max == rmax && st[c].arg < token)) { rmax = st[c].max; token = st[c].arg; }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float om = __shfl_xor_sync(0xffffffffu, rmax, o);
+        const int32_t ot = __shfl_xor_sync(0xffffffffu, token, o);
+        if (om > rmax || (om == rmax && ot < token)) { rmax = om; token = ot; }
+    }
     double total = 0.0;
-    for (int c = 0; c < n_chunks; ++c) total += st[c].sum * exp((double)st[c].max - (double)rmax);
+    for (int c = lane; c < n_chunks; c += 32) total += st[c].sum * exp((double)st[c].max - (double)rmax);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+    if (lane != 0) return;
     const double rlog = log(total);
     if (token < 0 || token >= V) token = 0;      // a row of NaNs has no arg-max: stay inside the row
     const float * raw = raw_logits + (size_t)row * V;
@@ -574,20 +995,34 @@ __global__ void greedy_finish_kernel(const float * __restrict__ raw_logits, int 
 
 } // namespace
 
-size_t sample_scratch_bytes(int n_vocab, int n_rows) { return (size_t)n_rows * ((n_vocab + kChunk - 1) / kChunk) * sizeof(ChunkStat); }
+size_t sample_scratch_bytes(int n_vocab, int n_rows, bool candidates) {
+    const size_t chunks = (size_t)n_rows * ((n_vocab + kChunk - 1) / kChunk);
+    return chunks * (sizeof(ChunkStat) + (candidates ? kChunkCands * sizeof(Cand) : 0));
+}
+
+bool sample_chunked(int n_vocab, bool v2, int top_k, float min_p, float top_p, uint32_t n_top) {
+    if ((n_vocab + kChunk - 1) / kChunk > kThreads) return false;
+    if (v2 && top_k > 0 && top_k < n_vocab) return top_k <= kMaxNeed;
+    return top_p >= 1.0f && !(v2 && min_p > 0.0f) && n_top <= (uint32_t)kMaxNeed;
+}
 
 void launch_sample(const float * raw_logits, float * work_logits, int n_vocab, int n_rows, const SampleDesc * desc, const LogitEdit * edits,
-                   const uint32_t * masks, SampleOut * out,
-                   int32_t * top_ids, float * top_logprobs, int top_stride, int n_greedy_fast, void * scratch, cudaStream_t stream) {
+                   const uint32_t * masks, SampleOut * out, int32_t * top_ids, float * top_logprobs, int top_stride, int n_greedy_fast, int n_chunked,
+                   void * scratch, cudaStream_t stream) {
     if (n_rows <= 0) return;
-    if (n_greedy_fast < n_rows)
-        sample_kernel<<<n_rows, kThreads, 0, stream>>>(raw_logits, work_logits, n_vocab, desc, edits, masks, out, top_ids, top_logprobs, top_stride);
-    if (n_greedy_fast > 0) {
-        const int n_chunks = (n_vocab + kChunk - 1) / kChunk;
-        ChunkStat * stats = static_cast<ChunkStat *>(scratch);
-        greedy_chunk_kernel<<<dim3(n_chunks, n_rows), kChunkThreads, 0, stream>>>(raw_logits, n_vocab, desc, stats, n_chunks);
-        greedy_finish_kernel<<<n_rows, 32, 0, stream>>>(raw_logits, n_vocab, desc, stats, n_chunks, out, top_ids, top_logprobs, top_stride);
+    const int n_chunks = (n_vocab + kChunk - 1) / kChunk;
+    ChunkStat * stats = static_cast<ChunkStat *>(scratch);
+    Cand * cands = reinterpret_cast<Cand *>(stats + (size_t)n_rows * n_chunks);
+    if (n_greedy_fast + n_chunked > 0)
+        sample_chunk_kernel<<<dim3(n_chunks, n_rows), kChunkThreads, 0, stream>>>(raw_logits, n_vocab, desc, edits, stats, cands, n_chunks, top_stride);
+    if (n_greedy_fast < n_rows) {
+        static PerDeviceOnce configured;   // function attributes are per device
+        if (configured.first()) cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RowShared));
+        sample_kernel<<<n_rows, kThreads, n_chunked ? sizeof(RowShared) : 0, stream>>>(raw_logits, work_logits, n_vocab, desc, edits, masks, stats, cands,
+                                                                                       n_chunks, out, top_ids, top_logprobs, top_stride);
     }
+    if (n_greedy_fast > 0)
+        greedy_finish_kernel<<<n_rows, 32, 0, stream>>>(raw_logits, n_vocab, desc, stats, n_chunks, out, top_ids, top_logprobs, top_stride);
 }
 
 } // namespace rb200

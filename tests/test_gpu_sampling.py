@@ -1,0 +1,76 @@
+"""Sampling rows served from per-chunk results (4096 logits a chunk): truncated and untruncated draws, edits, top lists,
+against the CPU restatement on the same logits, at vocabulary sizes around the chunk's edges."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _transformed(logits, sp):
+    """The logits the draw works on: bias, then top_k (ties: lowest ids), then min_p."""
+    l = logits.copy()
+    for token, bias in sp.logit_bias:
+        l[token] = np.float32(l[token] + np.float32(bias))
+    if 0 < sp.top_k < l.size:
+        order = np.argsort(-l, kind="stable")
+        l[order[sp.top_k :]] = -np.inf
+    if sp.min_p > 0:
+        l[l < l.max() + np.log(np.float32(sp.min_p))] = -np.inf
+    return l
+
+
+@pytest.mark.parametrize("vocab", [260, 4096, 4097, 12293])
+def test_chunked_rows_match_the_restatement(rb, oracle, models, vocab):
+    path = models(f"sampling_{vocab}", arch="llama", layers=1, d=256, heads=4, kv_heads=4, ff=256, vocab=vocab, dtype="q8_0", seed=9)
+    far = vocab - 1
+    options = [dict(temperature=1.0), dict(temperature=0.7), dict(temperature=1.3, logit_bias=[(5, 2.0), (far, 3.5)]), dict(top_k=2),
+               dict(top_k=20), dict(temperature=0.8, top_k=40, top_p=0.95, min_p=0.05), dict(temperature=1.2, top_k=128, top_p=0.5),
+               dict(top_k=7, logit_bias=[(far, 4.0), (17, -50.0)]), dict(top_k=129), dict(top_k=20, top_p=1e-4), dict(top_k=1, logit_bias=[(far, 9.0)])]
+    with rb.Engine(str(path), rb.EngineConfig(n_ctx=1024, n_seq_max=len(options), n_batch=256, n_ubatch=256)) as engine:
+        out = rb.StepOutput()
+        prompt = np.arange(3, 12).tolist()
+        for draw in range(6):
+            params = [rb.SamplingParamsV2(seed=50 + i, **o) for i, o in enumerate(options)]
+            rows = [rb.StepRow(i, i, prompt if draw == 0 else [out.row(i).token], 0 if draw == 0 else len(prompt) + draw - 1, True, sp, 5, True)
+                    for i, sp in enumerate(params)]
+            engine.step(rows, out)
+            for i, sp in enumerate(params):
+                logits, o = engine.last_logits(i), out.row(i)
+                l = _transformed(logits, sp)
+                want, margin = oracle.sample_philox(l, sp.temperature, sp.top_p, sp.seed, draw)
+                # the two sums differ in the order of their additions: a draw within 1e-9 of a border may fall on either side
+                assert o.token == want or margin < 1e-9, (sp, o.token, want, margin)
+                assert o.logprob == pytest.approx(float(oracle.token_logprob(logits, o.token)), abs=2e-6)
+                p = np.exp((l.astype(np.float64) - l.max()) / sp.temperature)
+                if sp.top_p < 1 or sp.top_k == 1:
+                    order = np.argsort(-p, kind="stable")
+                    keep = 1 if sp.top_k == 1 else int(np.searchsorted(np.cumsum(p[order]), sp.top_p * p.sum()) + 1)
+                    mask = np.zeros(p.size)
+                    mask[order[:keep]] = 1
+                    p = p * mask
+                p /= p.sum()
+                assert o.sampled_logprob == pytest.approx(np.log(p[o.token]), abs=1e-5)
+                ids, lps = out.top(i)
+                order = np.lexsort((np.arange(p.size), -np.where(p > 0, l, -np.inf)))
+                assert list(ids) == order[:5].tolist()
+                with np.errstate(divide="ignore"):
+                    np.testing.assert_allclose(lps, np.log(p[order[:5]]), atol=1e-5)
+
+
+def test_rows_of_ties_take_the_lowest_ids(rb, models):
+    """A model of zero weights: every logit is equal, so the candidate lists overflow and the general passes serve the row."""
+    path = models("sampling_ties", arch="llama", layers=1, d=256, heads=4, kv_heads=4, ff=256, vocab=9000, dtype="f32", std=0, seed=1)
+    with rb.Engine(str(path), rb.EngineConfig(n_ctx=256, n_seq_max=2, n_batch=64, n_ubatch=64)) as engine:
+        out = rb.StepOutput()
+        seen = set()
+        for trial in range(12):
+            for slot in (0, 1):
+                engine.seq_rm(slot)
+            rows = [rb.StepRow(10 + trial, 0, [5, 6], 0, True, rb.SamplingParamsV2(top_k=5, seed=trial), 3, True),
+                    rb.StepRow(100 + trial, 1, [5], 0, True, rb.SamplingParamsV2(top_k=0, seed=trial))]
+            engine.step(rows, out)
+            seen.add(out.row(0).token)
+            assert 0 <= out.row(0).token < 5 and list(out.top(0)[0]) == [0, 1, 2]
+            assert out.row(0).sampled_logprob == pytest.approx(np.log(0.2), abs=1e-6)
+            assert out.row(0).logprob == pytest.approx(-np.log(9000), abs=1e-6)
+        assert len(seen) > 1
