@@ -110,6 +110,7 @@ struct StepProfiler {
 // Device storage of one SplitAct for up to `rows` rows of `ld` columns.
 struct SplitBuffer {
     DeviceBuffer<__half> store;
+    std::vector<CUtensorMap> box_maps;
     SplitAct view;
     void ensure(size_t rows, size_t ld) {
         if (ld % 32 != 0) return;
@@ -120,7 +121,8 @@ struct SplitBuffer {
         view.sum_hi = store.ptr + 2 * main;
         view.sum_lo = store.ptr + 2 * main + sums + 32;
         view.ld = (int)ld;
-        split_act_encode_maps(view, rows);
+        box_maps.resize(16);
+        split_act_encode_maps(view, rows, box_maps.data());
     }
     const SplitAct * get() const { return view.hi ? &view : nullptr; }
 };

@@ -113,12 +113,12 @@ __global__ void __launch_bounds__(STHREADS, 1) gemm_q4k_stream_kernel(const uint
                 // K step ks = sub-block ks / 2 of the half, word ks % 2: elements 4 (2 tq + ks % 2) .. + 3 of the sub-block
                 const int e = (ks >> 1) * 32 + 4 * (2 * tq + (ks & 1));
                 const uint2 vh = *reinterpret_cast<const uint2 *>(src_a + row + e);
-                bh[ks][0] = __byte_perm(vh.x, vh.y, 0x5410);     // elements 0, 2
-                bh[ks][1] = __byte_perm(vh.x, vh.y, 0x7632);     // elements 1, 3
+                bh[ks][0] = vh.x;     // elements 0, 1: bytes 0 and 2 of the word (the tiled copy's order is 0, 2, 1, 3)
+                bh[ks][1] = vh.y;     // elements 2, 3
                 if (!PACK4) {
                     const uint2 vl = *reinterpret_cast<const uint2 *>(X.lo + row + e);
-                    bl[ks][0] = __byte_perm(vl.x, vl.y, 0x5410);
-                    bl[ks][1] = __byte_perm(vl.x, vl.y, 0x7632);
+                    bl[ks][0] = vl.x;
+                    bl[ks][1] = vl.y;
                 }
             }
             if (!PACK4 || g < 4) {

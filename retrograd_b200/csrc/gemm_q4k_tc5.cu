@@ -62,22 +62,35 @@ constexpr int STAGE_BYTES = 2 * B_BYTES;          // activation tiles hi and lo;
 #endif
 constexpr int GROUPS = RB200_TC5_GROUPS;          // producer groups of four warps
 constexpr int EPI_WARP0 = 4 * GROUPS, MMA_WARP = EPI_WARP0 + 8;
-constexpr int N_WARPS = MMA_WARP + 1;
+constexpr int TMA_WARP = MMA_WARP + 1;
+constexpr int N_WARPS = TMA_WARP + 1;
 constexpr int THREADS = N_WARPS * 32;
 constexpr int TMEM_COLS = 512;
 constexpr int TMEM_A = 256;                    // column offsets: accumulators at 0 and 128, then the A slots
 static_assert(STAGES >= 2 && STAGES <= 8, "the A slots share 256 tensor-memory columns");
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /* alignment slack */ + 256 /* barriers */;
 
-__device__ __forceinline__ void nibbles_times_scale(uint32_t word, int hi, __half2 sc2, __half2 off2, uint32_t & out01, uint32_t & out23) {
-    const uint32_t v = hi ? (word >> 4) : word;
-    uint32_t a = (v & 0x000F000Fu) | 0x64006400u;
-    uint32_t b = ((v >> 8) & 0x000F000Fu) | 0x64006400u;
-    const __half2 ha = __hfma2(*reinterpret_cast<__half2 *>(&a), sc2, off2);
-    const __half2 hb = __hfma2(*reinterpret_cast<__half2 *>(&b), sc2, off2);
-    const uint32_t ua = *reinterpret_cast<const uint32_t *>(&ha), ub = *reinterpret_cast<const uint32_t *>(&hb);
-    out01 = __byte_perm(ua, ub, 0x5410);
-    out23 = __byte_perm(ua, ub, 0x7632);
+__device__ __forceinline__ __half2 as_half2(uint32_t v) { return *reinterpret_cast<const __half2 *>(&v); }
+__device__ __forceinline__ uint32_t as_u32(__half2 v) { return *reinterpret_cast<const uint32_t *>(&v); }
+
+// One sub-block of a group: the low (HIGH = false) or high nibbles of its eight words -> 32 exact integers sc * q as f16,
+// two per register in K order. Integer and conversion instructions issue at half rate or less, so an f16 pair costs one
+// masking instruction and one fused multiply-add: the tiled copy keeps the bytes of a word in the order 0, 2, 1, 3, a
+// masked nibble under the exponent of 1024 is 1024 + q (16 q for the high nibbles), and (1024 + q) sc - 1024 sc resp.
+// (1024 + 16 q) sc / 16 - 64 sc are exact.
+template <bool HIGH>
+__device__ __forceinline__ void nibbles_times_scale(const uint32_t (&word)[8], __half2 scale, __half2 offset, uint32_t (&out)[16]) {
+    constexpr uint32_t mask = HIGH ? 0x00F000F0u : 0x000F000Fu;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        out[2 * i] = as_u32(__hfma2(as_half2((word[i] & mask) | 0x64006400u), scale, offset));
+        out[2 * i + 1] = as_u32(__hfma2(as_half2(((word[i] >> 8) & mask) | 0x64006400u), scale, offset));
+    }
+}
+
+// bytes 0, 1, 2, 3 of every word -> 0, 2, 1, 3
+__device__ __forceinline__ uint4 q4k_interleave_bytes(uint4 v) {
+    return make_uint4(__byte_perm(v.x, 0, 0x3120), __byte_perm(v.y, 0, 0x3120), __byte_perm(v.z, 0, 0x3120), __byte_perm(v.w, 0, 0x3120));
 }
 
 // grid (super-blocks, row tiles), 128 threads: thread p moves the 144-byte block of row p
@@ -98,8 +111,8 @@ __global__ void q4k_retile_kernel(const uint8_t * __restrict__ rows, uint32_t n_
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         uint4 * q = reinterpret_cast<uint4 *>(dst + q4k_tile_group_offset(p, r));
-        q[0] = v[1 + 2 * r];
-        q[1] = v[2 + 2 * r];
+        q[0] = q4k_interleave_bytes(v[1 + 2 * r]);
+        q[1] = q4k_interleave_bytes(v[2 + 2 * r]);
     }
 }
 
@@ -109,7 +122,7 @@ __global__ void q4k_retile_kernel(const uint8_t * __restrict__ rows, uint32_t n_
 template <bool RESIDUAL, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, 1) gemm_q4k_tc5_kernel(const uint8_t * __restrict__ W, int n_in, int n_out, int row_bytes,
                                                                   const __grid_constant__ SplitAct X, int T, float * __restrict__ Y, int ldy, const float * __restrict__ bias,
-                                                                  const float * __restrict__ residual, int ldr, int * __restrict__ error_flag,
+                                                                  const float * __restrict__ residual, int ldr, int * __restrict__ error_flag, int tn,
                                                                   int sb_per_split, float * __restrict__ partial) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t * smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -124,7 +137,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_q4k_tc5_kernel(const uint8_t 
     volatile int * abort_flag = reinterpret_cast<volatile int *>(tmem_word + 1);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int m0 = blockIdx.y * BM, t0 = blockIdx.x * BN;   // token tiles vary fastest: CTAs in flight share a weight tile in L2
+    const int m0 = blockIdx.y * BM, t0 = blockIdx.x * tn;   // token tiles vary fastest: CTAs in flight share a weight tile in L2
     // split-K: blockIdx.z owns super-blocks [sb0, sb0 + n_sb) of the row and writes a partial result
     const int n_sb_all = n_in / 256;
     const int sb0 = SPLIT ? blockIdx.z * sb_per_split : 0;
@@ -134,7 +147,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_q4k_tc5_kernel(const uint8_t 
 
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) {
-            tc5::mbar_init(full_bar(s), 4);     // the producer group's warps; the TMA bytes are tracked as transactions
+            tc5::mbar_init(full_bar(s), 5);     // the producer group's warps and the fetching warp, whose bytes are tracked as transactions
             tc5::mbar_init(empty_bar(s), 1);
         }
         for (int b = 0; b < 2; ++b) {
@@ -157,94 +170,96 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_q4k_tc5_kernel(const uint8_t 
         // (the tiled layout is zero-padded to whole row tiles: every row p exists)
         const uint8_t * tile_base = W + ((size_t)blockIdx.y * n_sb_all + sb0) * kQ4kTileBytes;
         const int t = t0 + p;
-        const bool t_valid = t < T;
+        const bool t_valid = p < tn && t < T;
         // Raw block bytes are prefetched into registers two own stages ahead, so the HBM latency of
         // the weights never holds a pipeline slot; a slot is only held for the L2 latency of the
         // activation copy, which overlaps the decode.
         struct Raw { uint4 hdr, q0, q1; };
-        auto prefetch = [&](int it, Raw & raw) {
-            if (it >= n_it) return;
-            const int sb = it / 5, r = it % 5;
-            const uint8_t * blk = tile_base + (size_t)sb * kQ4kTileBytes;
-            raw.hdr = *reinterpret_cast<const uint4 *>(blk + q4k_tile_hdr_offset(p));      // consecutive threads, consecutive bytes
-            if (r < 4) {
-                const uint4 * qs = reinterpret_cast<const uint4 *>(blk + q4k_tile_group_offset(p, r));
+        // the group's next prefetch: stage `ahead_r` of super-block `ahead_sb` at `ahead`
+        int ahead_r = group, ahead_sb = 0;
+        const uint8_t * ahead = tile_base;
+        static_assert(GROUPS < 5, "a group's next stage lies in the same or the next super-block");
+        auto prefetch = [&](Raw & raw) {
+            if (ahead_sb >= n_sb) return;
+            raw.hdr = *reinterpret_cast<const uint4 *>(ahead + q4k_tile_hdr_offset(p));      // consecutive threads, consecutive bytes
+            if (ahead_r < 4) {
+                const uint4 * qs = reinterpret_cast<const uint4 *>(ahead + q4k_tile_group_offset(p, ahead_r));
                 raw.q0 = qs[0];
                 raw.q1 = qs[1];
             } else {
                 raw.q0 = raw.q1 = make_uint4(0, 0, 0, 0);
                 if (t_valid) {
-                    raw.q0 = *reinterpret_cast<const uint4 *>(X.sum_hi + (size_t)t * n_sub + (sb0 + sb) * 8);
-                    raw.q1 = *reinterpret_cast<const uint4 *>(X.sum_lo + (size_t)t * n_sub + (sb0 + sb) * 8);
+                    raw.q0 = *reinterpret_cast<const uint4 *>(X.sum_hi + (size_t)t * n_sub + (sb0 + ahead_sb) * 8);
+                    raw.q1 = *reinterpret_cast<const uint4 *>(X.sum_lo + (size_t)t * n_sub + (sb0 + ahead_sb) * 8);
                 }
             }
+            ahead_r += GROUPS;
+            if (ahead_r >= 5) {
+                ahead_r -= 5;
+                ++ahead_sb;
+                ahead += kQ4kTileBytes;
+            }
         };
+        int stage = group, parity = 1, r = group;
+        static_assert(GROUPS <= STAGES, "a group's next stage lies in the same or the next turn of the ring");
         // returns false when the pipeline was aborted
-        auto produce = [&](int it, Raw & raw) -> bool {
-            const int stage = it % STAGES, use = it / STAGES;
+        auto produce = [&](Raw & raw) -> bool {
             // warp-uniform outcome: the tensor-memory stores below are warp-collective
-            if (!__all_sync(0xffffffffu, tc5::mbar_wait(empty_bar(stage), (use & 1) ^ 1, abort_flag))) return false;
+            if (!__all_sync(0xffffffffu, tc5::mbar_wait(empty_bar(stage), parity, abort_flag))) return false;
             tc5::fence_after_sync();
-            const int sb = it / 5, r = it % 5;
-            uint8_t * bh_s = smem + stage * STAGE_BYTES;
             const uint32_t a_slot = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + TMEM_A + stage * 32;
             if (r < 4) {
-                if (p == 0) {
-                    // the activation tiles (hi and lo, 128 tokens x 64 columns each) arrive by TMA
-                    const uint32_t bh = smem_u32(bh_s), bl = bh + B_BYTES;
-                    tc5::mbar_expect_tx(full_bar(stage), 2 * B_BYTES);
-                    tc5::tma_load_2d(bh, &X.map_hi, (sb0 + sb) * 256 + r * 64, t0, full_bar(stage));
-                    tc5::tma_load_2d(bl, &X.map_lo, (sb0 + sb) * 256 + r * 64, t0, full_bar(stage));
-                }
-                // 64 weights -> 32 columns of f16 pairs in K order: low nibbles (columns 0..31 of the group), then high
-                uint32_t out[32];
-#pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    uint32_t sc, mn;
-                    q4k_scale_min_regs(raw.hdr, r * 2 + half, sc, mn);
-                    const __half2 sc2 = __half2half2(__ushort2half_rn((unsigned short)sc));
-                    const __half2 off2 = __half2half2(__float2half_rn(-1024.0f * (float)sc));
-                    uint32_t * o = out + half * 16;
-                    nibbles_times_scale(raw.q0.x, half, sc2, off2, o[0], o[1]);
-                    nibbles_times_scale(raw.q0.y, half, sc2, off2, o[2], o[3]);
-                    nibbles_times_scale(raw.q0.z, half, sc2, off2, o[4], o[5]);
-                    nibbles_times_scale(raw.q0.w, half, sc2, off2, o[6], o[7]);
-                    nibbles_times_scale(raw.q1.x, half, sc2, off2, o[8], o[9]);
-                    nibbles_times_scale(raw.q1.y, half, sc2, off2, o[10], o[11]);
-                    nibbles_times_scale(raw.q1.z, half, sc2, off2, o[12], o[13]);
-                    nibbles_times_scale(raw.q1.w, half, sc2, off2, o[14], o[15]);
-                }
-                tc5::tmem_st32(a_slot, out);
-                prefetch(it + 2 * GROUPS, raw);
+                // 64 weights -> 32 columns of f16 pairs in K order: low nibbles (columns 0..31 of the group), then high.
+                // The group's two scales are bytes 2 r and 2 r + 1 of the unpacked eight; a byte under the exponent of
+                // 1024 becomes an f16 with one permute and one subtraction.
+                const uint32_t scales = (r < 2 ? raw.hdr.y & 0x3F3F3F3Fu : (raw.hdr.w & 0x0F0F0F0Fu) | ((raw.hdr.y >> 2) & 0x30303030u)) >> ((r & 1) * 16);
+                const __half2 k1024 = __float2half2_rn(1024.f);
+                const __half2 sc_lo = __hsub2(as_half2(__byte_perm(scales, 0x64646464u, 0x4040)), k1024);
+                const __half2 sc_hi = __hsub2(as_half2(__byte_perm(scales, 0x64646464u, 0x4141)), k1024);
+                const uint32_t words[8] = {raw.q0.x, raw.q0.y, raw.q0.z, raw.q0.w, raw.q1.x, raw.q1.y, raw.q1.z, raw.q1.w};
+                uint32_t out[16];
+                nibbles_times_scale<false>(words, sc_lo, __hmul2(sc_lo, __float2half2_rn(-1024.f)), out);
+                tc5::tmem_st16_nowait(a_slot, out);
+                nibbles_times_scale<true>(words, __hmul2(sc_hi, __float2half2_rn(0.0625f)), __hmul2(sc_hi, __float2half2_rn(-64.f)), out);
+                tc5::tmem_st16_nowait(a_slot + 16, out);
+                prefetch(raw);
+                tc5::tmem_wait_st();
             } else {
                 // minimum-term stage: A = [-rho*m_0..7 hi | lo], B tiles [sum_hi | sum_hi] and [sum_lo | sum_lo]
-                const __half2 dd = *reinterpret_cast<const __half2 *>(&raw.hdr.x);
+                const __half2 dd = as_half2(raw.hdr.x);
                 const float d = __low2float(dd), dmin = __high2float(dd);
                 const float nrho = d != 0.f ? -dmin / d : 0.f;
+                const uint32_t mins[2] = {raw.hdr.z & 0x3F3F3F3Fu, ((raw.hdr.w >> 4) & 0x0F0F0F0Fu) | ((raw.hdr.z >> 2) & 0x30303030u)};
                 uint32_t mw[8];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    uint32_t s0, n0, s1, n1;
-                    q4k_scale_min_regs(raw.hdr, 2 * q, s0, n0);
-                    q4k_scale_min_regs(raw.hdr, 2 * q + 1, s1, n1);
-                    const float v0 = nrho * (float)n0, v1 = nrho * (float)n1;
-                    const __half h0 = __float2half_rn(v0), h1 = __float2half_rn(v1);
-                    const __half2 hi2 = __halves2half2(h0, h1);
-                    const __half2 lo2 = __halves2half2(__float2half_rn(v0 - __half2float(h0)), __float2half_rn(v1 - __half2float(h1)));
-                    mw[q] = *reinterpret_cast<const uint32_t *>(&hi2);
-                    mw[q + 4] = *reinterpret_cast<const uint32_t *>(&lo2);
+                    // a byte in the low mantissa bits of 2^23 reads as 2^23 + m
+                    const float m0 = __uint_as_float(__byte_perm(mins[q >> 1], 0x4B000000u, 0x7540u | (2 * q & 3))) - 8388608.f;
+                    const float m1 = __uint_as_float(__byte_perm(mins[q >> 1], 0x4B000000u, 0x7540u | ((2 * q + 1) & 3))) - 8388608.f;
+                    const float v0 = nrho * m0, v1 = nrho * m1;
+                    const __half2 hi2 = __floats2half2_rn(v0, v1);
+                    const __half2 lo2 = __floats2half2_rn(v0 - __low2float(hi2), v1 - __high2float(hi2));
+                    mw[q] = as_u32(hi2);
+                    mw[q + 4] = as_u32(lo2);
                 }
                 tc5::tmem_st8(a_slot, mw);
-                *reinterpret_cast<uint4 *>(bh_s + swz(p, 0)) = raw.q0;
-                *reinterpret_cast<uint4 *>(bh_s + swz(p, 1)) = raw.q0;
-                *reinterpret_cast<uint4 *>(bh_s + B_BYTES + swz(p, 0)) = raw.q1;
-                *reinterpret_cast<uint4 *>(bh_s + B_BYTES + swz(p, 1)) = raw.q1;
+                uint8_t * bh_s = smem + stage * STAGE_BYTES;
+                if (p < tn) {                          // the MMAs read no further rows of the tile
+                    *reinterpret_cast<uint4 *>(bh_s + swz(p, 0)) = raw.q0;
+                    *reinterpret_cast<uint4 *>(bh_s + swz(p, 1)) = raw.q0;
+                    *reinterpret_cast<uint4 *>(bh_s + B_BYTES + swz(p, 0)) = raw.q1;
+                    *reinterpret_cast<uint4 *>(bh_s + B_BYTES + swz(p, 1)) = raw.q1;
+                }
                 tc5::fence_proxy_async();
-                prefetch(it + 2 * GROUPS, raw);
+                prefetch(raw);
             }
             tc5::fence_before_sync();
             __syncwarp();
             if (lane == 0) tc5::mbar_arrive(full_bar(stage));
+            r += GROUPS;
+            if (r >= 5) r -= 5;
+            stage += GROUPS;
+            if (stage >= STAGES) { stage -= STAGES; parity ^= 1; }
             return true;
         };
         Raw raw0, raw1;
@@ -253,13 +268,38 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_q4k_tc5_kernel(const uint8_t 
         // one - so such a stage among the first two waits its turn.
         static_assert(GROUPS < 4, "the first stage of every group must be a weight stage");
         const bool sums_first = (group + GROUPS) % 5 == 4;
-        prefetch(group, raw0);
-        if (!sums_first) prefetch(group + GROUPS, raw1);
+        prefetch(raw0);
+        if (!sums_first) prefetch(raw1);
         asm volatile("griddepcontrol.wait;" ::: "memory");
-        if (sums_first) prefetch(group + GROUPS, raw1);
+        if (sums_first) prefetch(raw1);
         for (int it = group; it < n_it; it += 2 * GROUPS) {
-            if (!produce(it, raw0)) break;
-            if (it + GROUPS < n_it && !produce(it + GROUPS, raw1)) break;
+            if (!produce(raw0)) break;
+            if (it + GROUPS < n_it && !produce(raw1)) break;
+        }
+    } else if (warp == TMA_WARP) {
+        // ------------------------------------------------------------------ activation tiles
+        // hi and lo, tn tokens x 64 columns each, by TMA as soon as the slot is free (a producer that did this on the side
+        // fetched late and held its own decode up); the minimum-term stage's tiles are the producers'
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        int stage = 0, parity = 1, x = sb0 * 256;
+        bool alive = true;
+        for (int sb = 0; sb < n_sb && alive; ++sb) {
+            for (int r = 0; r < 5; ++r) {
+                if (!__all_sync(0xffffffffu, tc5::mbar_wait(empty_bar(stage), parity, abort_flag))) { alive = false; break; }
+                if (lane == 0) {
+                    if (r < 4) {
+                        const uint32_t bh = smem_base + stage * STAGE_BYTES;
+                        tc5::mbar_arrive_expect_tx(full_bar(stage), tn * 256u);
+                        tc5::tma_load_2d(bh, &X.map_hi, x + r * 64, t0, full_bar(stage));
+                        tc5::tma_load_2d(bh + B_BYTES, &X.map_lo, x + r * 64, t0, full_bar(stage));
+                    } else {
+                        tc5::mbar_arrive(full_bar(stage));
+                    }
+                }
+                __syncwarp();
+                if (++stage == STAGES) { stage = 0; parity ^= 1; }
+            }
+            x += 256;
         }
     } else if (warp == MMA_WARP) {
         // ------------------------------------------------------------------ MMA issue
@@ -270,8 +310,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_q4k_tc5_kernel(const uint8_t 
             // uniform. (With a single thread inside a divergent branch the issuing thread - not the tensor
             // pipe - set the pace: 0.94 -> 0.81 ms on 28 672 x 4096 x 2048.) Descriptors are built once; a
             // stage costs an add per operand and the MMAs themselves.
-            // the step's last token tile only pays for the columns it has, in whole MMA widths of 16
-            const uint32_t idesc = tc5::instr_desc_f16(BM, min(BN, (T - t0 + 15) & ~15));
+            const uint32_t idesc = tc5::instr_desc_f16(BM, tn);
             const uint64_t desc0 = tc5::smem_desc_sw128(smem_base);
             const uint32_t desc_lo0 = (uint32_t)desc0, desc_hi = (uint32_t)(desc0 >> 32);
             const uint32_t a_slot0 = tmem_base + TMEM_A;
@@ -333,13 +372,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_q4k_tc5_kernel(const uint8_t 
             tc5::fence_after_sync();
             const uint32_t t_main = t_lane + buf * 128;
 #pragma unroll
-            for (int c = 0; c < 4; c += 2) {
-                float v[16], w[16];
-                tc5::tmem_ld16x2(t_main + c * 16, t_main + (c + 1) * 16, v, w);
+            for (int c = 0; c < 64; c += 8) {
+                if (colhalf * 64 + c < tn) {           // warp-uniform: columns that the MMAs do not write stay unread
+                    float v[8];
+                    tc5::tmem_ld8(t_main + c, v);
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    acc[c * 16 + i] += d * v[i];
-                    acc[(c + 1) * 16 + i] += d * w[i];
+                    for (int i = 0; i < 8; ++i) acc[c + i] += d * v[i];
                 }
             }
             tc5::fence_before_sync();
@@ -348,10 +386,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_q4k_tc5_kernel(const uint8_t 
         }
         if (alive && o_valid) {
             const float b = bias ? bias[o] : 0.f;
+            const int t_end = min(T, t0 + tn);
 #pragma unroll
             for (int i = 0; i < 64; ++i) {
                 const int t = t0 + colhalf * 64 + i;
-                if (t < T) {
+                if (t < t_end) {
                     if (SPLIT) {
                         partial[((size_t)blockIdx.z * T + t) * n_out + o] = acc[i];      // bias and residual are added by the finish kernel
                     } else {
@@ -396,22 +435,37 @@ EncodeFn tensor_map_encoder() {
 
 bool tensor_maps_available() { return tensor_map_encoder() != nullptr; }
 
-bool split_act_encode_maps(SplitAct & s, size_t rows) {
+bool split_act_encode_maps(SplitAct & s, size_t rows, CUtensorMap * box_maps) {
     const EncodeFn encode = tensor_map_encoder();
     s.has_maps = 0;
+    s.box_maps = nullptr;
     if (!encode || !s.hi || s.ld % 64 != 0 || rows == 0) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)s.ld, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)s.ld * sizeof(__half)};
-    const cuuint32_t box[2] = {64, 128};
     const cuuint32_t elem[2] = {1, 1};
-    for (int which = 0; which < 2; ++which) {
-        const CUresult r = encode(which ? &s.map_lo : &s.map_hi, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, which ? (void *)s.lo : (void *)s.hi, dims,
-                                  strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) return false;
+    for (cuuint32_t height = box_maps ? 16 : 128; height <= 128; height += 16) {
+        const cuuint32_t box[2] = {64, height};
+        CUtensorMap maps[2];
+        for (int which = 0; which < 2; ++which) {
+            const CUresult r = encode(&maps[which], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, which ? (void *)s.lo : (void *)s.hi, dims, strides, box, elem,
+                                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+            if (r != CUDA_SUCCESS) return false;
+            if (box_maps) box_maps[(height / 16 - 1) * 2 + which] = maps[which];
+        }
+        s.map_hi = maps[0];
+        s.map_lo = maps[1];
     }
     s.has_maps = 1;
+    s.box_maps = box_maps;
     return true;
+}
+
+SplitAct split_act_with_boxes(const SplitAct & x, int height) {
+    SplitAct r = x;
+    r.map_hi = x.box_maps[(height / 16 - 1) * 2];
+    r.map_lo = x.box_maps[(height / 16 - 1) * 2 + 1];
+    return r;
 }
 
 bool attention_maps_encode(AttentionMaps & maps, const __half * k, const __half * v, int head_dim, uint64_t rows) {
@@ -433,7 +487,7 @@ bool attention_maps_encode(AttentionMaps & maps, const __half * k, const __half 
 }
 
 bool gemm_q4k_tc5_supported(const WeightView & w, const SplitAct & x) {
-    return w.type == GGML_Q4_K && w.tiled && w.tc5_exact && w.n_in % 256 == 0 && x.hi && x.ld == (int)w.n_in && x.has_maps;
+    return w.type == GGML_Q4_K && w.tiled && w.tc5_exact && w.n_in % 256 == 0 && x.hi && x.ld == (int)w.n_in && x.box_maps;
 }
 
 bool q4k_min_fold_ok(const uint8_t * blocks, size_t n_blocks) {
@@ -478,7 +532,11 @@ void launch_gemm_q4k_tc5(const WeightView & w, const SplitAct & x, int n_tokens,
     if ((size_t)splits * n_tokens * w.n_out > scratch_floats) splits = 1;
     const int sb_per_split = (n_sb + splits - 1) / splits;
     float * partial = splits > 1 ? scratch : nullptr;
-    const dim3 grid((n_tokens + BN - 1) / BN, (w.n_out + BM - 1) / BM, splits);
+    // token tiles of equal height, so that no tile waits for a wider one, and activation boxes of just that height
+    const int token_tiles = (n_tokens + BN - 1) / BN;
+    const int tn = ((n_tokens + token_tiles - 1) / token_tiles + 15) & ~15;
+    const SplitAct xs = split_act_with_boxes(x, tn);
+    const dim3 grid(token_tiles, (w.n_out + BM - 1) / BM, splits);
     // the kernel may start (barriers, tensor-memory allocation, first weight loads) while the stream's
     // earlier kernels drain; every role waits on the device before it touches activations or outputs
     cudaLaunchConfig_t cfg = {};
@@ -494,14 +552,14 @@ void launch_gemm_q4k_tc5(const WeightView & w, const SplitAct & x, int n_tokens,
     const float * no_residual = nullptr;
     if (splits > 1) {
         // bias and residual are the finish kernel's
-        cudaLaunchKernelEx(&cfg, gemm_q4k_tc5_kernel<false, true>, w.tiled, (int)w.n_in, (int)w.n_out, (int)w.row_bytes, x, n_tokens, y, ldy, bias,
-                           no_residual, 0, error_flag, sb_per_split, partial);
+        cudaLaunchKernelEx(&cfg, gemm_q4k_tc5_kernel<false, true>, w.tiled, (int)w.n_in, (int)w.n_out, (int)w.row_bytes, xs, n_tokens, y, ldy, bias,
+                           no_residual, 0, error_flag, tn, sb_per_split, partial);
     } else if (residual) {
-        cudaLaunchKernelEx(&cfg, gemm_q4k_tc5_kernel<true, false>, w.tiled, (int)w.n_in, (int)w.n_out, (int)w.row_bytes, x, n_tokens, y, ldy, bias, residual,
-                           ldr, error_flag, sb_per_split, partial);
+        cudaLaunchKernelEx(&cfg, gemm_q4k_tc5_kernel<true, false>, w.tiled, (int)w.n_in, (int)w.n_out, (int)w.row_bytes, xs, n_tokens, y, ldy, bias, residual,
+                           ldr, error_flag, tn, sb_per_split, partial);
     } else {
-        cudaLaunchKernelEx(&cfg, gemm_q4k_tc5_kernel<false, false>, w.tiled, (int)w.n_in, (int)w.n_out, (int)w.row_bytes, x, n_tokens, y, ldy, bias,
-                           no_residual, 0, error_flag, sb_per_split, partial);
+        cudaLaunchKernelEx(&cfg, gemm_q4k_tc5_kernel<false, false>, w.tiled, (int)w.n_in, (int)w.n_out, (int)w.row_bytes, xs, n_tokens, y, ldy, bias,
+                           no_residual, 0, error_flag, tn, sb_per_split, partial);
     }
     if (splits > 1) launch_gemm_stream_finish(scratch, splits, (int)w.n_out, n_tokens, n_tokens, y, ldy, bias, residual, ldr, stream, tail);
 }

@@ -34,7 +34,8 @@ struct WeightView {
 // quarter holds, for its rows, the 32 nibble bytes of 64-column groups 0 and 1 (2 x 1024 bytes), then
 // the 32 block headers of 16 bytes (d, dmin, packed scales), then groups 2 and 3: either half of the
 // columns together with the headers is one contiguous 2560-byte range, and a warp that takes one row
-// per lane reads consecutive bytes.
+// per lane reads consecutive bytes. The nibble bytes of every 32-bit word are kept in the order 0, 2, 1, 3, so that the
+// nibbles of neighbouring columns lie 16 bits apart, where an f16 pair has them.
 constexpr size_t kQ4kTileBytes = 18432;
 constexpr size_t kQ4kQuarterBytes = 4608;
 __host__ __device__ inline size_t q4k_tile_hdr_offset(int p) { return (size_t)(p >> 5) * kQ4kQuarterBytes + 2048 + (size_t)(p & 31) * 16; }
@@ -142,14 +143,19 @@ struct SplitAct {
     __half * sum_lo = nullptr;
     int ld = 0;
     int has_maps = 0;
+    // Host memory of the owner: the descriptors below for boxes of 16, 32 .. 128 rows, [height / 16 - 1][hi, lo]; null when
+    // only the ones below exist.
+    const CUtensorMap * box_maps = nullptr;
     // TMA descriptors over hi and lo ([rows][ld] f16, boxes of 64 columns x 128 rows, 128-byte swizzle)
     alignas(64) CUtensorMap map_hi;
     alignas(64) CUtensorMap map_lo;
 };
 
-// Fills the TMA descriptors of `s` for `rows` rows; returns false when the driver entry point is
-// unavailable (the kernels that need them are then not selected).
-bool split_act_encode_maps(SplitAct & s, size_t rows);
+// Fills the TMA descriptors of `s` for `rows` rows, and with `box_maps` (16 of them) those of every box height; returns
+// false when the driver entry point is unavailable (the kernels that need them are then not selected).
+bool split_act_encode_maps(SplitAct & s, size_t rows, CUtensorMap * box_maps = nullptr);
+// `x` with map_hi and map_lo for boxes of `height` rows (a multiple of 16, at most 128).
+SplitAct split_act_with_boxes(const SplitAct & x, int height);
 
 // The step of the layer that consumes a streaming GEMM's result, done by the GEMM's finish kernel on the
 // row it has just summed (one launch and one pass over the row less):

@@ -252,5 +252,18 @@ __device__ __forceinline__ void tmem_ld16x2(uint32_t taddr_a, uint32_t taddr_b, 
     }
 }
 
+// Eight consecutive f32 columns of this thread's TMEM lane, for callers with no registers for more.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&a)[8]) {
+    uint32_t r[8];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+        "tcgen05.wait::ld.sync.aligned;\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+        : "r"(taddr)
+        : "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) a[i] = __uint_as_float(r[i]);
+}
+
 } // namespace tc5
 } // namespace rb200

@@ -46,6 +46,22 @@ def test_q4k_tcgen05_gemm_against_float64(rb, oracle, n_out, n_in, T):
     assert err < 4e-6
 
 
+@pytest.mark.parametrize("T", [1, 16, 17, 113, 128, 129, 160, 161, 257, 385])
+def test_q4k_tcgen05_token_tiles_of_every_height(rb, oracle, T):
+    """Token tiles are of equal height, in steps of 16 (16, 32, 128, 80, 96 and 112 tokens here), each with activation boxes of
+    its own height; 150 row tiles keep the reduction whole, 150 x 128 rows less three leave the last one ragged."""
+    n_out, n_in = 150 * 128 - 3, 512
+    rng = np.random.default_rng(T)
+    raw = _q4k_matrix(rb, rng, 256, n_in)
+    raw = np.tile(raw, n_out // 256 + 1)[: n_out * (n_in // 256) * 144]
+    x = rng.normal(0, 1.5, (T, n_in)).astype(np.float32)
+    w = oracle.dequantize_row(oracle.T_Q4_K, raw, n_out * n_in).reshape(n_out, n_in).astype(np.float64)
+    want = x.astype(np.float64) @ w.T
+    got, _ = rb.op_gemm(12, raw, n_out, n_in, x, path=4)
+    # the bound of the other shapes: f32 sums of exact products
+    assert float(np.abs(got - want).max()) / float(np.abs(want).max()) < 4e-6
+
+
 @pytest.mark.parametrize("n_out,n_in,T", [(256, 512, 1), (384, 1024, 3), (200, 768, 8), (512, 2816, 5), (1040, 4096, 8), (128, 14336, 2)])
 def test_q4k_streaming_gemm_against_float64(rb, oracle, n_out, n_in, T):
     """The weight-streaming kernel for at most eight tokens: exact products, ragged row counts, and
