@@ -10,25 +10,30 @@
 // matrix qualifies when every super-block has d != 0 or dmin * m == 0, and |rho * m| stays far inside
 // the f16 range (q4k_min_fold_ok, checked once at load); other matrices take the mma.sync kernel.
 //
-// One CTA computes 128 weight rows x 128 tokens. Warp roles (21 warps):
-//   0-11       three producer groups of four warps, taking pipeline stages in turn (the decode is a
-//              dependent instruction chain per thread: with two groups the producers were busy 92 % of
-//              the time and the issuing warp waited for them a third of it); thread p decodes the 64 weights of
+// One CTA computes 128 weight rows x up to 128 tokens. Token tiles are of equal height, a multiple of 16. Warp roles
+// (22 warps):
+//   0-11       three producer groups of four warps, taking pipeline stages in turn; thread p decodes the 64 weights of
 //              row p and stores them into lane p of the stage's A slot in TENSOR MEMORY (the MMA reads
-//              its A operand from there, so shared memory carries the activations only); one thread
-//              of the group fetches the two activation tiles (hi and lo) with TMA, whose bytes
-//              complete on the stage's barrier;
+//              its A operand from there, so shared memory carries the activations only);
 //   20         walks the pipeline as a whole warp (uniform address arithmetic); one elected lane issues
-//              the MMAs (M 128, N 128, K 16) and commits them to the stage's "empty" barrier, and per
+//              the MMAs (M 128, N the tile's height, K 16) and commits them to the stage's "empty" barrier, and per
 //              super-block to the accumulator's "full" barrier;
+//   21         fetches the two activation tiles (hi and lo) of a free slot with TMA, whose bytes
+//              complete on the stage's barrier;
 //   12-19      epilogue: each thread owns one weight row and 64 token columns, pulls the TMEM
 //              accumulator of a finished super-block with tcgen05.ld and folds it, times d, into its
 //              f32 running sums while the tensor cores already work on the next super-block in the
 //              other buffer.
 // Tensor memory (512 columns): two accumulators (2 x 128) and the pipeline's A slots of 32 columns
-// (128 rows x 64 f16). The pipeline is five stages deep (shared memory: 5 x 32 KB of activation
-// tiles); measured on 28 672 x 4096 x 2048 with three producer groups: three stages 0.88 ms, four
-// 0.77, five 0.75-0.76, six 0.79, seven 0.81.
+// (128 rows x 64 f16). The pipeline is five stages deep (shared memory: 5 x 32 KB of activation tiles).
+// Measured on 28 672 x 4096 (us at 17 / 30 / 60 / 128 / 203 / 437 / 1781 tokens): 66 / 68 / 70 / 75 / 131 / 224 / 730 with
+// producers that permuted, converted and fetched and boxes of 128 tokens whatever the tile's height; 59 / 61 / 63 / 71 /
+// 121 / 210 / 701 with the cheaper decode and the fetching warp; 57 / 57 / 59 / 66 / 117 / 201 / 691 with the tile's own
+// height. What bounds it: at 1781 tokens the activations' 32 KB a stage out of L2 (621 us when only a quarter is fetched);
+// below 128 tokens none of decode, MMAs, loads or copies alone (each left out: 52 to 57 us), but the roles' hand-over
+// and about 10 us per tile from its launch to its last store. Two producer groups instead of three (before the last step):
+// 64 / 65 / 68 / 72 / 126 / 213 / 691. A persistent form with equal shares per SM was slower throughout (919 us at 1781):
+// its longer code made the warps wait for instructions.
 // A super-block is five pipeline stages: four of 64 columns each (eight MMAs: hi and lo), then one
 // that carries the minimum term as two K=16 steps (A = [-rho*m hi | -rho*m lo], B = [sum_hi | sum_hi],
 // then the same A with B = [sum_lo | sum_lo]).
