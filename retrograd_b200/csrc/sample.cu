@@ -252,18 +252,19 @@ __device__ __forceinline__ int needed(const SampleDesc & d, int V, int top_strid
 // of the log-sum (one per logit), not by memory: 257 rows of 201 088 logits take 130 us, 1.6 TB/s.
 // Candidates: with `need` values wanted of the whole row, the need-th largest of the 256 per-thread maxima is a lower
 // bound of the chunk's need-th largest value; everything at or above it goes to the list (a few more than `need`).
+// CHUNKED: the step has rows that are served from candidate lists. A step of greedy rows alone takes the form without them,
+// whose smaller register and shared-memory need lets more blocks hide the exponentials' latency.
+template <bool CHUNKED>
 __global__ void __launch_bounds__(kChunkThreads) sample_chunk_kernel(const float * __restrict__ raw_logits, int V, const SampleDesc * __restrict__ descs,
                                                                      const LogitEdit * __restrict__ edits, ChunkStat * __restrict__ stats,
                                                                      Cand * __restrict__ cands, int n_chunks, int top_stride) {
     const int row = blockIdx.y, chunk = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const SampleDesc d = descs[row];
-    if (!(d.flags & (kFlagGreedyFast | kFlagChunked))) return;
+    if (!(d.flags & (CHUNKED ? kFlagGreedyFast | kFlagChunked : kFlagGreedyFast))) return;
     constexpr int PER = kChunk / kChunkThreads;
     __shared__ float s_max[kChunkThreads / 32];
     __shared__ int32_t s_arg[kChunkThreads / 32];
     __shared__ double s_sum[kChunkThreads / 32];
-    __shared__ float s_val[kChunk];
-    __shared__ int s_count;
     const float * l = raw_logits + (size_t)row * V;
     const int base = chunk * kChunk;
     float v[PER];
@@ -320,7 +321,9 @@ __global__ void __launch_bounds__(kChunkThreads) sample_chunk_kernel(const float
     st.tsum = st.sum;
     st.count = 0;
     st.pad[0] = st.pad[1] = st.pad[2] = 0;
-    if (d.flags & kFlagChunked) {
+    if (CHUNKED && (d.flags & kFlagChunked)) {
+        __shared__ float s_val[CHUNKED ? kChunk : 1];
+        __shared__ int s_count;
         const uint32_t n_edits = (d.flags & kFlagV2) ? d.edit_end - d.edit_begin : 0u;
         if (n_edits) {
 #pragma unroll
@@ -1013,8 +1016,10 @@ void launch_sample(const float * raw_logits, float * work_logits, int n_vocab, i
     const int n_chunks = (n_vocab + kChunk - 1) / kChunk;
     ChunkStat * stats = static_cast<ChunkStat *>(scratch);
     Cand * cands = reinterpret_cast<Cand *>(stats + (size_t)n_rows * n_chunks);
-    if (n_greedy_fast + n_chunked > 0)
-        sample_chunk_kernel<<<dim3(n_chunks, n_rows), kChunkThreads, 0, stream>>>(raw_logits, n_vocab, desc, edits, stats, cands, n_chunks, top_stride);
+    if (n_chunked > 0)
+        sample_chunk_kernel<true><<<dim3(n_chunks, n_rows), kChunkThreads, 0, stream>>>(raw_logits, n_vocab, desc, edits, stats, cands, n_chunks, top_stride);
+    else if (n_greedy_fast > 0)
+        sample_chunk_kernel<false><<<dim3(n_chunks, n_rows), kChunkThreads, 0, stream>>>(raw_logits, n_vocab, desc, edits, stats, cands, n_chunks, top_stride);
     if (n_greedy_fast < n_rows) {
         static PerDeviceOnce configured;   // function attributes are per device
         if (configured.first()) cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RowShared));
