@@ -37,6 +37,7 @@ namespace {
 
 constexpr int BM = 128;
 constexpr int TMEM_COLS = 512;
+constexpr int kMaxSplits = 8, kMinSplitStages = 8;
 
 // A producer warp reads the 32 x 68 bytes of its rows' stage segments as 544 consecutive-per-row words - lane after
 // lane along a row, so a load instruction touches two or three rows instead of 32 - and hands every lane its own
@@ -70,11 +71,13 @@ __device__ __forceinline__ void int8x4_to_half2(uint32_t u, __half2 & a, __half2
     b = __hsub2(*reinterpret_cast<__half2 *>(&ub), off);
 }
 
-template <int BN, bool RESIDUAL>
+// SPLIT: blockIdx.z owns a range of the reduction's stages and writes its result to `partial`; the finish kernel of the
+// streaming GEMMs adds them in order, with bias and residual.
+template <int BN, bool RESIDUAL, bool SPLIT>
 __global__ void __launch_bounds__(Shape<BN>::THREADS, 1) gemm_q8_0_tc5_kernel(const uint8_t * __restrict__ W, int n_in, int n_out, int row_bytes,
                                                                    const __grid_constant__ SplitAct X, int T, float * __restrict__ Y, int ldy,
                                                                    const float * __restrict__ bias, const float * __restrict__ residual, int ldr,
-                                                                   int * __restrict__ error_flag) {
+                                                                   int * __restrict__ error_flag, int it_per_split, float * __restrict__ partial) {
     using S = Shape<BN>;
     constexpr int STAGES = S::STAGES, B_BYTES = S::B_BYTES, STAGE_BYTES = S::STAGE_BYTES;
     constexpr int GROUPS = S::GROUPS, EPI_WARP0 = S::EPI_WARP0, MMA_WARP = S::MMA_WARP;
@@ -91,7 +94,8 @@ __global__ void __launch_bounds__(Shape<BN>::THREADS, 1) gemm_q8_0_tc5_kernel(co
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int m0 = blockIdx.y * BM, t0 = blockIdx.x * BN;   // token tiles vary fastest: CTAs in flight share a weight tile in L2
-    const int n_it = n_in / 64;
+    const int it0 = SPLIT ? blockIdx.z * it_per_split : 0;
+    const int n_it = SPLIT ? min(n_in / 64, it0 + it_per_split) - it0 : n_in / 64;
     // a tile with fewer tokens than columns only pays for the columns it has, in whole MMA widths of 16
     const int mma_n = min(BN, (T - t0 + 15) & ~15);
 
@@ -119,7 +123,7 @@ __global__ void __launch_bounds__(Shape<BN>::THREADS, 1) gemm_q8_0_tc5_kernel(co
         // values. They are prefetched two own stages ahead, so the HBM latency never holds a pipeline slot.
         struct Raw { uint32_t w[17]; };
         // word i of the warp's 544 (i = 32 k + lane) is word i % 17 of row i / 17
-        const uint8_t * warp_rows = W + (size_t)(m0 + (warp & 3) * 32) * row_bytes;
+        const uint8_t * warp_rows = W + (size_t)(m0 + (warp & 3) * 32) * row_bytes + (size_t)it0 * 68;
         const int rows_left = n_out - (m0 + (warp & 3) * 32);
         uint32_t * exchange = reinterpret_cast<uint32_t *>(smem + S::ROWS_OFF + warp * kRowExchangeBytes);
         auto prefetch = [&](int it, Raw & raw) {
@@ -169,8 +173,8 @@ __global__ void __launch_bounds__(Shape<BN>::THREADS, 1) gemm_q8_0_tc5_kernel(co
                 tc5::mbar_expect_tx(full_bar(stage), 2 * B_BYTES);
 #pragma unroll
                 for (int box = 0; box < BN / 128; ++box) {
-                    tc5::tma_load_2d(bh + box * 16384, &X.map_hi, it * 64, t0 + box * 128, full_bar(stage));
-                    tc5::tma_load_2d(bl + box * 16384, &X.map_lo, it * 64, t0 + box * 128, full_bar(stage));
+                    tc5::tma_load_2d(bh + box * 16384, &X.map_hi, (it0 + it) * 64, t0 + box * 128, full_bar(stage));
+                    tc5::tma_load_2d(bl + box * 16384, &X.map_lo, (it0 + it) * 64, t0 + box * 128, full_bar(stage));
                 }
             }
             const uint32_t a_slot = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + S::TMEM_A + stage * 64;
@@ -250,6 +254,11 @@ __global__ void __launch_bounds__(Shape<BN>::THREADS, 1) gemm_q8_0_tc5_kernel(co
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
                         const int ta = t0 + col0 + c + i, tb = ta + 16;
+                        if (SPLIT) {
+                            if (ta < T) partial[((size_t)blockIdx.z * T + ta) * n_out + o] = v[i];
+                            if (tb < T) partial[((size_t)blockIdx.z * T + tb) * n_out + o] = w[i];
+                            continue;
+                        }
                         if (ta < T) {
                             float r = v[i] + b;
                             if (RESIDUAL) r += residual[(size_t)ta * ldr + o];
@@ -275,15 +284,16 @@ __global__ void __launch_bounds__(Shape<BN>::THREADS, 1) gemm_q8_0_tc5_kernel(co
     if (tid == 0 && *abort_flag) atomicExch(error_flag, 1);
 }
 
-template <int BN, bool RESIDUAL>
+template <int BN, bool RESIDUAL, bool SPLIT>
 void launch_one(const WeightView & w, const SplitAct & x, int n_tokens, float * y, int ldy, const float * bias, const float * residual, int ldr,
-                int * error_flag, cudaStream_t stream) {
+                int * error_flag, int splits, float * partial, cudaStream_t stream) {
     static PerDeviceOnce configured;   // function attributes are per device
-    if (configured.first()) cudaFuncSetAttribute(gemm_q8_0_tc5_kernel<BN, RESIDUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<BN>::SMEM_BYTES);
+    if (configured.first())
+        cudaFuncSetAttribute(gemm_q8_0_tc5_kernel<BN, RESIDUAL, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<BN>::SMEM_BYTES);
     // the kernel may start (barriers, tensor-memory allocation, first weight loads) while the stream's
     // earlier kernels drain; every role waits on the device before it touches activations or outputs
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((n_tokens + BN - 1) / BN, (w.n_out + BM - 1) / BM);
+    cfg.gridDim = dim3((n_tokens + BN - 1) / BN, (w.n_out + BM - 1) / BM, splits);
     cfg.blockDim = dim3(Shape<BN>::THREADS);
     cfg.dynamicSmemBytes = Shape<BN>::SMEM_BYTES;
     cfg.stream = stream;
@@ -292,8 +302,57 @@ void launch_one(const WeightView & w, const SplitAct & x, int n_tokens, float * 
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, gemm_q8_0_tc5_kernel<BN, RESIDUAL>, w.data, (int)w.n_in, (int)w.n_out, (int)w.row_bytes, x, n_tokens, y, ldy, bias, residual,
-                       ldr, error_flag);
+    const int n_it = (int)w.n_in / 64;
+    cudaLaunchKernelEx(&cfg, gemm_q8_0_tc5_kernel<BN, RESIDUAL, SPLIT>, w.data, (int)w.n_in, (int)w.n_out, (int)w.row_bytes, x, n_tokens, y, ldy, bias,
+                       residual, ldr, error_flag, (n_it + splits - 1) / splits, partial);
+}
+
+template <int BN>
+void launch_form(const WeightView & w, const SplitAct & x, int n_tokens, float * y, int ldy, const float * bias, const float * residual, int ldr,
+                 int * error_flag, int splits, float * partial, cudaStream_t stream) {
+    if (splits > 1) launch_one<BN, false, true>(w, x, n_tokens, y, ldy, nullptr, nullptr, 0, error_flag, splits, partial, stream);
+    else if (residual) launch_one<BN, true, false>(w, x, n_tokens, y, ldy, bias, residual, ldr, error_flag, 1, nullptr, stream);
+    else launch_one<BN, false, false>(w, x, n_tokens, y, ldy, bias, nullptr, 0, error_flag, 1, nullptr, stream);
+}
+
+struct Plan {
+    bool wide;
+    int splits;
+};
+
+// The form and the number of splits with the shortest estimated time, in cycles, for whole waves of one CTA per SM.
+// 256-token tiles halve the decode work per product (measured per 64-column stage: about 1800 cycles at N = 256, where the
+// twelve MMAs take 1536, and 1300 at N = 128, where the producers set the pace; narrower MMAs do not help the producers). A
+// split costs the write and the read of its partial results (about 2000 bytes per cycle) and the finish kernel a launch;
+// every wave pays for its CTAs' beginning and end. Unsplit, 4096 x 14 336 took 153 us and 4096 x 4096 50 us from 24 tokens to
+// 512 (32 row tiles on 148 SMs); with the splits a step of 320 rows over eight layers of the 8B shape went from 8437 to 7879 us,
+// two steps of 24 rows over four layers of the 20B-class mixture of experts from 4725 to 4354 us.
+Plan plan_of(uint32_t n_out, uint32_t n_in, int n_tokens, int n_sm) {
+    static const int forced = [] {          // RB200_Q8_TC5_TILE=128|256 pins the form (measurements)
+        const char * env = std::getenv("RB200_Q8_TC5_TILE");
+        return env ? std::atoi(env) : 0;
+    }();
+    const int n_it = (int)n_in / 64, row_tiles = (int)((n_out + BM - 1) / BM);
+    Plan best{false, 1};
+    long long best_cycles = -1;
+    for (int wide = 0; wide < 2; ++wide) {
+        if (wide && (n_tokens <= 128 || forced == 128)) continue;
+        if (!wide && n_tokens > 128 && forced == 256) continue;
+        const long long tiles = (long long)row_tiles * ((n_tokens + (wide ? 255 : 127)) / (wide ? 256 : 128));
+        for (int splits = 1; splits <= kMaxSplits && (splits == 1 || n_it / splits >= kMinSplitStages); ++splits) {
+            const int per_split = (n_it + splits - 1) / splits;
+            if ((n_it + per_split - 1) / per_split != splits) continue;      // an empty last range
+            if (splits > 1 && tiles * splits > n_sm) break;                  // a split that does not fit one wave gains too little for its traffic
+            const long long waves = (tiles * splits + n_sm - 1) / n_sm;
+            long long cycles = waves * ((long long)per_split * (wide ? 1800 : 1300) + 6000);
+            if (splits > 1) cycles += 6000 + (long long)splits * n_tokens * n_out * 8 / 2000;
+            if (best_cycles < 0 || cycles < best_cycles) {
+                best_cycles = cycles;
+                best = Plan{wide != 0, splits};
+            }
+        }
+    }
+    return best;
 }
 
 } // namespace
@@ -315,29 +374,18 @@ bool gemm_q8_0_tc5_supported(const WeightView & w, const SplitAct & x) {
            x.ld == (int)w.n_in && x.has_maps;
 }
 
+size_t gemm_q8_0_tc5_scratch_floats(uint32_t n_out, uint32_t n_in, int n_tokens, int n_sm) {
+    const int splits = plan_of(n_out, n_in, n_tokens, n_sm).splits;
+    return splits > 1 ? (size_t)splits * n_tokens * n_out : 0;
+}
+
 void launch_gemm_q8_0_tc5(const WeightView & w, const SplitAct & x, int n_tokens, float * y, int ldy, const float * bias, const float * residual,
-                          int ldr, int * error_flag, int n_sm, cudaStream_t stream) {
+                          int ldr, int * error_flag, float * scratch, int n_sm, cudaStream_t stream, const FinishTail * tail) {
     if (n_tokens <= 0) return;
-    // 256-token tiles halve the decode work per product, but the grid is whole waves of one CTA per SM: the form
-    // with the shorter estimated time wins (measured per 64-column stage: about 1800 cycles at N = 256, where the
-    // twelve MMAs take 1536, and 1300 at N = 128, where the producers set the pace)
-    const int row_tiles = (int)((w.n_out + BM - 1) / BM);
-    const long long waves_wide = ((long long)row_tiles * ((n_tokens + 255) / 256) + n_sm - 1) / n_sm;
-    const long long waves_narrow = ((long long)row_tiles * ((n_tokens + 127) / 128) + n_sm - 1) / n_sm;
-    bool wide = n_tokens > 128 && waves_wide * 1800 < waves_narrow * 1300;
-    static const int forced = [] {          // RB200_Q8_TC5_TILE=128|256 pins the form (measurements)
-        const char * env = std::getenv("RB200_Q8_TC5_TILE");
-        return env ? std::atoi(env) : 0;
-    }();
-    if (forced == 128) wide = false;
-    if (forced == 256 && n_tokens > 128) wide = true;
-    if (wide) {
-        if (residual) launch_one<256, true>(w, x, n_tokens, y, ldy, bias, residual, ldr, error_flag, stream);
-        else launch_one<256, false>(w, x, n_tokens, y, ldy, bias, nullptr, 0, error_flag, stream);
-    } else {
-        if (residual) launch_one<128, true>(w, x, n_tokens, y, ldy, bias, residual, ldr, error_flag, stream);
-        else launch_one<128, false>(w, x, n_tokens, y, ldy, bias, nullptr, 0, error_flag, stream);
-    }
+    const Plan plan = plan_of(w.n_out, w.n_in, n_tokens, n_sm);
+    if (plan.wide) launch_form<256>(w, x, n_tokens, y, ldy, bias, residual, ldr, error_flag, plan.splits, scratch, stream);
+    else launch_form<128>(w, x, n_tokens, y, ldy, bias, residual, ldr, error_flag, plan.splits, scratch, stream);
+    if (plan.splits > 1) launch_gemm_stream_finish(scratch, plan.splits, (int)w.n_out, n_tokens, n_tokens, y, ldy, bias, residual, ldr, stream, tail);
 }
 
 } // namespace rb200

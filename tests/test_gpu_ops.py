@@ -164,3 +164,18 @@ def test_mxfp4_grouped_tcgen05_gemm_against_float64(rb, oracle, n_expert, n_out,
         worst = max(worst, float(np.abs(got[rows] - want).max()) / float(np.abs(want).max()))
     print(f"mxfp4 grouped tcgen05 {n_expert}x{n_out}x{n_in} rows={counts}: rel err {worst:.2e}")
     assert worst < 2e-5         # one tensor-core accumulator over the whole row, as for Q8_0 above
+
+
+@pytest.mark.parametrize("n_out,n_in,T", [(128, 1024, 17), (200, 1216, 33), (256, 4096, 128), (384, 2880, 129), (2048, 1088, 300)])
+def test_q8_0_tcgen05_splits_of_the_reduction(rb, oracle, n_out, n_in, T):
+    """Few output tiles: the reduction is cut into ranges of stages (16 to 64 of them here, a short last range in the second,
+    fourth and fifth shape), in both tile forms; bounds as for the whole reduction."""
+    rng = np.random.default_rng(n_out + n_in + T)
+    w = rng.normal(0, 0.02, (n_out, n_in)).astype(np.float32)
+    raw = np.frombuffer(b"".join(rb.quantize_row(8, w[r]) for r in range(n_out)), dtype=np.uint8)
+    x = rng.normal(0, 1.5, (T, n_in)).astype(np.float32)
+    wd = oracle.dequantize_row(oracle.T_Q8_0, raw, n_out * n_in).reshape(n_out, n_in).astype(np.float64)
+    want = x.astype(np.float64) @ wd.T
+    got, _ = rb.op_gemm(8, raw, n_out, n_in, x, path=4)
+    scale = np.abs(wd).max(axis=1) * np.abs(x).max() * np.sqrt(n_in)
+    assert float((np.abs(got - want) / scale[None, :]).max()) < 2e-5
