@@ -5,7 +5,8 @@
 // into chunks of 4096 logits that separate blocks read ONCE (sample_chunk_kernel: maximum, sum of exponentials, and the
 // chunk's candidates for the largest `need` values), and one block per row finishes from the chunks' results
 // (sample_kernel, row_from_chunks). The general passes remain for rows the chunks cannot serve: grammar masks, forced
-// tokens, a nucleus over the whole vocabulary, top_k above kMaxNeed, and rows whose ties overflow a candidate list.
+// tokens, a nucleus over the whole vocabulary, top_k above kMaxNeed, rows whose ties overflow a candidate list, and rows with
+// a NaN, an infinite maximum or a negative zero among their candidates.
 //
 // What is reproduced from the reference's CPU oracle
 // (crates/retrograd-ffi/runtime/src/retro_gen_core.cpp:41-51,103-225,718-875,2942-2985):
@@ -69,8 +70,11 @@ struct Shared {
     unsigned long long ullval2;
 };
 
+// Integers in the order of the floats; a positive NaN comes above them all. The bits are moved out by hand: as a plain cast the
+// compiler may set the sign bit with a float negation, which gives NaNs other bits (they then ranked with the negative zero).
 __device__ __forceinline__ uint32_t order_key(float f) {
-    const uint32_t u = __float_as_uint(f);
+    uint32_t u;
+    asm("mov.b32 %0, %1;" : "=r"(u) : "f"(f));
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
@@ -351,6 +355,7 @@ __global__ void __launch_bounds__(kChunkThreads) sample_chunk_kernel(const float
                 const uint32_t t = bound | (1u << bit);
                 if (__syncthreads_count(mine >= t) >= need) bound = t;
             }
+            if (bound == order_key(0.f)) bound = order_key(-0.f);       // equal values are handed on together
             if (tid == 0) s_count = 0;
             __syncthreads();
             Cand * list = cands + ((size_t)row * n_chunks + chunk) * kChunkCands;
@@ -385,8 +390,8 @@ struct RowShared {
     int32_t rarg, targ, n_keep, token, chunk, n_list;
 };
 
-// The last step of a row whose chunks hold everything it needs; false when they do not (more ties than the lists take):
-// the caller then runs the general passes. Follows the general kernel's rules line by line (the comments there).
+// The last step of a row whose chunks hold everything it needs; false when they do not (more ties than the lists take, a
+// NaN, an infinite maximum, a negative zero among the candidates): the caller then runs the general passes. Follows the general kernel's rules line by line (the comments there).
 __device__ bool row_from_chunks(Shared & sh, RowShared & rs, const float * __restrict__ raw, int V, const SampleDesc & d, const LogitEdit * __restrict__ edits,
                                 const ChunkStat * __restrict__ st, const Cand * __restrict__ cands, int n_chunks, SampleOut * __restrict__ out,
                                 int32_t * __restrict__ top_ids, float * __restrict__ top_lps, int top_stride) {
@@ -421,12 +426,15 @@ __device__ bool row_from_chunks(Shared & sh, RowShared & rs, const float * __res
         }
         if (lane == 0) { rs.rmax = m; rs.rarg = a; rs.tmax = em; rs.targ = ea; rs.rtotal = total; rs.total = ttotal; }
     }
+    __syncthreads();
+    // a NaN or an infinite maximum (of the raw row, or by its edits) makes a sum a NaN: the general passes have their rules for those
+    if (!(rs.rtotal < INFINITY) || !(fabsf(rs.tmax) < INFINITY) || (!cut && !(rs.total < INFINITY))) return false;
     // ---- the largest `need` values, exactly
     int n_list = 0;
     if (need > 0) {
         int32_t n_cand;
         int32_t mine = 0;
-        bool over = false;
+        bool over = false, unordered = false;
         if (tid < n_chunks) { mine = st[tid].count; over = mine > kChunkCands; }
         const int32_t first = block_exclusive_scan_int(sh, mine, &n_cand);
         rs.offset[tid] = first;
@@ -437,9 +445,12 @@ __device__ bool row_from_chunks(Shared & sh, RowShared & rs, const float * __res
                 const Cand e = cands[(size_t)c * kChunkCands + i];
                 rs.cv[at + i] = e.v;
                 rs.cid[at + i] = e.id;
+                // the selection below goes by order_key, the order of the list by value: they differ for a NaN (edits can make one of
+                // a finite row) and for the two zeros
+                unordered = unordered || e.v != e.v || __float_as_uint(e.v) == 0x80000000u;
             }
         }
-        __syncthreads();
+        if (__syncthreads_or(unordered)) return false;
         uint32_t key[kRowCands / kThreads];
         const int slots = (n_cand + kThreads - 1) / kThreads;
 #pragma unroll

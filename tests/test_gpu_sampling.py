@@ -74,3 +74,89 @@ def test_rows_of_ties_take_the_lowest_ids(rb, models):
             assert out.row(0).sampled_logprob == pytest.approx(np.log(0.2), abs=1e-6)
             assert out.row(0).logprob == pytest.approx(-np.log(9000), abs=1e-6)
         assert len(seen) > 1
+
+
+@pytest.mark.parametrize("vocab", [260, 9000])
+def test_rows_with_a_nan_or_an_infinity_keep_the_general_rules(rb, oracle, models, tmp_path, vocab):
+    """Output rows of NaN and of infinities: a NaN counts against top_k (its order key is above every number) and is never drawn
+    or listed; an infinite logit leaves no probability. The order of the selection and that of the list differ for these."""
+    gguf = pytest.importorskip("gguf")
+    path = models(f"sampling_f32_{vocab}", arch="llama", layers=1, d=256, heads=4, kv_heads=4, ff=256, vocab=vocab, dtype="f32", seed=11)
+    for values in ({7: np.nan}, {7: np.nan, vocab - 2: np.nan, 130: np.nan}, {9: np.inf}, {9: -np.inf}):
+        file = tmp_path / "odd.gguf"
+        file.write_bytes(path.read_bytes())
+        reader = gguf.GGUFReader(str(file), "r+")
+        weight = next(t for t in reader.tensors if t.name == "output.weight").data
+        assert weight.shape == (vocab, 256)
+        for token, value in values.items():
+            weight[token, :] = 0
+            weight[token, 3] = value
+        weight.flush()
+        del reader, weight
+        options = [dict(top_k=5), dict(top_k=40, temperature=0.8), dict(), dict(top_k=1), dict(temperature=1.2)]
+        with rb.Engine(str(file), rb.EngineConfig(n_ctx=512, n_seq_max=8, n_batch=64, n_ubatch=64)) as engine:
+            out = rb.StepOutput()
+            for draw in range(4):
+                params = [rb.SamplingParamsV2(seed=30 + i, **o) for i, o in enumerate(options)]
+                engine.step([rb.StepRow(i, i, [5 + draw], draw, True, sp, 4, True) for i, sp in enumerate(params)], out)
+                for i, sp in enumerate(params):
+                    l, o = engine.last_logits(i), out.row(i)
+                    nan = np.isnan(l)
+                    assert nan.sum() == sum(np.isnan(v) for v in values.values()) and 0 <= o.token < vocab
+                    if nan.any():
+                        assert not nan[o.token] and np.isnan(o.logprob)
+                    if sp.top_k == 1 or np.nanmax(l) == np.inf:
+                        continue
+                    kept = l.copy()
+                    if sp.top_k:
+                        order = np.lexsort((np.arange(vocab), -np.where(nan, np.inf, l)))      # NaNs first
+                        kept[order[sp.top_k :]] = -np.inf
+                    want, margin = oracle.sample_philox(np.where(np.isnan(kept), np.float32(-np.inf), kept), sp.temperature, 1.0, sp.seed, draw)
+                    assert o.token == want or margin < 1e-9
+                    p = np.exp((kept.astype(np.float64) - np.nanmax(kept)) / sp.temperature)
+                    p /= np.nansum(p)
+                    assert o.sampled_logprob == pytest.approx(np.log(p[o.token]), abs=1e-5)
+                    n = int((p > 0).sum())
+                    best = np.lexsort((np.arange(vocab), -np.where(p > 0, kept, -np.inf)))[: min(n, 4)]
+                    assert list(out.top(i)[0][: len(best)]) == best.tolist()
+
+
+def test_edits_that_overflow_to_a_nan_keep_the_general_rules(rb, oracle, models):
+    """Each edit's parts are finite, the edited logit of a repeated token is not: (l + 3e38) / 1e-3 - 2 * 3e38 = inf - inf."""
+    path = models("sampling_edits", arch="llama", layers=1, d=256, heads=4, kv_heads=4, ff=256, vocab=6000, dtype="q8_0", seed=12)
+    with rb.Engine(str(path), rb.EngineConfig(n_ctx=512, n_seq_max=4, n_batch=64, n_ubatch=64)) as engine:
+        out = rb.StepOutput()
+        force = rb.SamplingParamsV2(top_k=1, logit_bias=[(4321, 100.0)])
+        for pos in range(2):
+            engine.step([rb.StepRow(0, 0, [5], pos, True, force)], out)
+            assert out.row(0).token == 4321
+        # the history is 4321 twice: its edit is a NaN, which takes one of the six places
+        sp = rb.SamplingParamsV2(top_k=6, seed=0, logit_bias=[(4321, 3e38), (17, 2.0)], repeat_penalty=1e-3, frequency_penalty=3e38)
+        engine.step([rb.StepRow(0, 0, [5], 2, True, sp, 8, True)], out)
+        l, o = engine.last_logits(0).copy(), out.row(0)
+        l[17] += np.float32(2.0)
+        l[4321] = -np.inf
+        order = np.argsort(-l, kind="stable")
+        l[order[5:]] = -np.inf
+        want, margin = oracle.sample_philox(l, 1.0, 1.0, 0, 2)
+        assert o.token == want or margin < 1e-9
+        p = np.exp(l.astype(np.float64) - l.max())
+        assert o.sampled_logprob == pytest.approx(np.log(p[o.token] / p.sum()), abs=1e-5) and np.isfinite(o.logprob)
+        # (the listing has probability zero after the five, in id order; the NaN is not in it)
+        assert list(out.top(0)[0]) == order[:5].tolist() + [i for i in range(9) if i not in order[:5]][:3]
+
+
+def test_negative_zeros_come_after_positive_ones_in_top_k(rb, models):
+    """Ten equal logits of zero, two of them turned negative by an edit that underflows: top_k counts the others first."""
+    path = models("sampling_zeros", arch="llama", layers=1, d=256, heads=4, kv_heads=4, ff=256, vocab=260, dtype="f32", std=0, seed=1)
+    zeros = [3, 4, 50, 51, 90, 91, 92, 200, 201, 259]
+    bias = [(i, -1.0) for i in range(260) if i not in zeros]
+    with rb.Engine(str(path), rb.EngineConfig(n_ctx=64, n_seq_max=2, n_batch=16, n_ubatch=16)) as engine:
+        out = rb.StepOutput()
+        for pos, token in enumerate((3, 50)):
+            engine.step([rb.StepRow(0, 0, [5], pos, True, rb.SamplingParamsV2(top_k=1, logit_bias=[(token, 5.0)]))], out)
+            assert out.row(0).token == token
+        sp = rb.SamplingParamsV2(top_k=9, logit_bias=bias + [(3, -1e-44), (50, -1e-44)], repeat_penalty=1e-3)
+        engine.step([rb.StepRow(0, 0, [5], 2, True, sp, 9, True)], out)
+        assert sorted(out.top(0)[0]) == sorted(i for i in zeros if i != 50)
+        assert out.row(0).sampled_logprob == pytest.approx(-np.log(9), abs=1e-6)
