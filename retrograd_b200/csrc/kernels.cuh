@@ -10,6 +10,8 @@
 
 #include <atomic>
 
+#include "sample_limits.hpp"
+
 namespace rb200 {
 
 // A weight matrix in device memory in its GGUF storage layout: n_out rows of n_in elements.
@@ -190,7 +192,6 @@ struct RowDesc {
 };
 
 constexpr uint32_t kSampleFlagChunked = 8u;     // the row is finished from the chunks' statistics and candidates
-constexpr int kSampleMaxNeed = 128;             // largest top_k (or, without top_k, n_top) such a row may have
 
 // Per sampling row parameters (64 bytes).
 struct SampleDesc {
@@ -478,9 +479,6 @@ void launch_lora_tc(const LoraGroup & group, const float * scales, int r_max, in
 // in `scratch` (sample_scratch_bytes(); `candidates`: some row asks for the largest values); `n_greedy_fast` is how
 // many rows carry bit 2.
 size_t sample_scratch_bytes(int n_vocab, int n_rows, bool candidates);
-// Whether a row with these options is served from per-chunk results (the caller then sets kSampleFlagChunked, provided the row
-// has no grammar mask and no forced token).
-bool sample_chunked(int n_vocab, bool v2, int top_k, float min_p, float top_p, uint32_t n_top);
 // `masks`: grammar rows carry in desc.pad[0] the word offset (plus one) of their one-bit-per-token mask; null without such rows.
 // `n_chunked`: rows that carry kSampleFlagChunked.
 void launch_sample(const float * raw_logits, float * work_logits, int n_vocab, int n_rows, const SampleDesc * desc, const LogitEdit * edits,

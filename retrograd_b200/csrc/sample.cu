@@ -5,8 +5,8 @@
 // into chunks of 4096 logits that separate blocks read ONCE (sample_chunk_kernel: maximum, sum of exponentials, and the
 // chunk's candidates for the largest `need` values), and one block per row finishes from the chunks' results
 // (sample_kernel, row_from_chunks). The general passes remain for rows the chunks cannot serve: grammar masks, forced
-// tokens, a nucleus over the whole vocabulary, top_k above kMaxNeed, rows whose ties overflow a candidate list, and rows with
-// a NaN, an infinite maximum or a negative zero among their candidates.
+// tokens, a nucleus over the whole vocabulary, a top_k whose candidates would not fit (sample_candidates_fit), rows whose
+// ties overflow a candidate list, and rows with a NaN, an infinite maximum or a negative zero among their candidates.
 //
 // What is reproduced from the reference's CPU oracle
 // (crates/retrograd-ffi/runtime/src/retro_gen_core.cpp:41-51,103-225,718-875,2942-2985):
@@ -30,13 +30,11 @@ namespace rb200 {
 
 namespace {
 
-constexpr int kThreads = 1024;
+constexpr int kThreads = kSampleRowThreads;
 constexpr uint32_t kFlagV2 = 1u, kFlagWantLogprob = 2u, kFlagGreedyFast = 4u, kFlagChunked = kSampleFlagChunked;
 
-constexpr int kChunk = 4096, kChunkThreads = 256;
-constexpr int kMaxNeed = kSampleMaxNeed;        // largest top_k / n_top served from candidate lists
-constexpr int kChunkCands = 256;                // candidates a chunk may hand on: about 174 of 4096 random values for need = 128
-constexpr int kRowCands = 4096;                 // candidates of a row the finishing block stages in shared memory
+constexpr int kChunk = kSampleChunk, kChunkThreads = kSampleChunkThreads;
+constexpr int kChunkCands = kSampleChunkCands, kRowCands = kSampleRowCands;
 constexpr int kListMax = 256;                   // values at or above the row's need-th largest (ties included)
 
 struct ChunkStat {
@@ -1012,12 +1010,6 @@ __global__ void greedy_finish_kernel(const float * __restrict__ raw_logits, int 
 size_t sample_scratch_bytes(int n_vocab, int n_rows, bool candidates) {
     const size_t chunks = (size_t)n_rows * ((n_vocab + kChunk - 1) / kChunk);
     return chunks * (sizeof(ChunkStat) + (candidates ? kChunkCands * sizeof(Cand) : 0));
-}
-
-bool sample_chunked(int n_vocab, bool v2, int top_k, float min_p, float top_p, uint32_t n_top) {
-    if ((n_vocab + kChunk - 1) / kChunk > kThreads) return false;
-    if (v2 && top_k > 0 && top_k < n_vocab) return top_k <= kMaxNeed;
-    return top_p >= 1.0f && !(v2 && min_p > 0.0f) && n_top <= (uint32_t)kMaxNeed;
 }
 
 void launch_sample(const float * raw_logits, float * work_logits, int n_vocab, int n_rows, const SampleDesc * desc, const LogitEdit * edits,

@@ -160,3 +160,25 @@ def test_negative_zeros_come_after_positive_ones_in_top_k(rb, models):
         engine.step([rb.StepRow(0, 0, [5], 2, True, sp, 9, True)], out)
         assert sorted(out.top(0)[0]) == sorted(i for i in zeros if i != 50)
         assert out.row(0).sampled_logprob == pytest.approx(-np.log(9), abs=1e-6)
+
+
+def test_top_k_at_the_limits_of_the_candidate_lists(rb, oracle, models):
+    """128 256 logits in 32 chunks: 96 candidates a chunk fit the row's list, 97 are left to the general passes, which take one
+    launch less. Both draw what the restatement draws."""
+    vocab = 128256
+    path = models("sampling_128256", arch="llama", layers=1, d=256, heads=4, kv_heads=4, ff=256, vocab=vocab, dtype="q8_0", seed=3)
+    launches = {}
+    with rb.Engine(str(path), rb.EngineConfig(n_ctx=1024, n_seq_max=4, n_batch=64, n_ubatch=64)) as engine:
+        out = rb.StepOutput()
+        for request, top_k in enumerate((64, 96, 97, 100, 128)):
+            for draw in range(3):
+                sp = rb.SamplingParamsV2(top_k=top_k, seed=request, temperature=1.5)
+                rows = [rb.StepRow(10 * request + slot, slot, [5 + draw + slot], 3 * request + draw, True, sp, 3, True) for slot in range(3)]
+                engine.step(rows, out)
+                launches[top_k] = engine.last_step_stats()[1]
+                for slot in range(3):
+                    l = _transformed(engine.last_logits(slot), sp)
+                    want, margin = oracle.sample_philox(l, sp.temperature, 1.0, sp.seed, draw)
+                    assert out.row(slot).token == want or margin < 1e-9
+                    assert list(out.top(slot)[0]) == np.argsort(-l, kind="stable")[:3].tolist()
+    assert launches[64] == launches[96] == launches[97] + 1 and launches[97] == launches[100] == launches[128]

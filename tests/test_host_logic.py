@@ -170,6 +170,13 @@ def test_kv_bookkeeping(tmp_path):
     assert out.returncode == 0, out.stderr
 
 
+def test_sampling_rows_are_admitted_to_candidate_lists_that_hold_them(tmp_path):
+    exe = tmp_path / "sample_limits_test"
+    subprocess.run(["g++", "-std=c++17", "-O2", "-o", str(exe), str(ROOT / "tests" / "cpp" / "sample_limits_test.cpp")], check=True)
+    out = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert out.returncode == 0, out.stdout + out.stderr
+
+
 def test_mxfp4_expert_blocks_recode_exactly_as_q8_0(rb, oracle):
     """The engine holds MXFP4 expert banks as Q8_0 for the tensor cores: the doubled E2M1 value as the int8,
     half the E8M0 scale as the f16 d. Every value must decode to the same f32; a scale an f16 cannot hold
