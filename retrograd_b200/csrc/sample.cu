@@ -704,17 +704,29 @@ __global__ void __launch_bounds__(kThreads) sample_kernel(const float * __restri
     // ---- the general passes: v2 rows transform a private copy of their row; v1 rows only read the raw one
     float * l = v2 ? work_logits + (size_t)row * V : const_cast<float *>(raw);
     __syncthreads();
-    if (v2) {
-        for (int i = tid; i < V; i += kThreads) l[i] = raw[i];        // (every pass below reads a thread's own elements or follows a barrier)
-        __syncthreads();
-    }
 
-    // ---- temperature-1 statistics of the raw row
+    // ---- temperature-1 statistics of the raw row; the copy is written on the way (the barriers of the arg-max publish it). Eight
+    // loads are in flight before the first store: one at a time, a row of 128 256 logits took 18 us longer.
     float rmax = -INFINITY;
     int32_t rarg = 0x7fffffff;
-    for (int i = tid; i < V; i += kThreads) {
-        const float v = l[i];
-        if (v > rmax) { rmax = v; rarg = i; }
+    if (v2) {
+        float * __restrict__ work = work_logits + (size_t)row * V;
+        for (int i0 = tid; i0 < V; i0 += 8 * kThreads) {
+            float v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = i0 + j * kThreads < V ? raw[i0 + j * kThreads] : -INFINITY;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int i = i0 + j * kThreads;
+                if (i < V) work[i] = v[j];
+                if (v[j] > rmax) { rmax = v[j]; rarg = i; }
+            }
+        }
+    } else {
+        for (int i = tid; i < V; i += kThreads) {
+            const float v = l[i];
+            if (v > rmax) { rmax = v; rarg = i; }
+        }
     }
     block_argmax(sh, rmax, rarg, rmax, rarg);
     double part = 0.0;

@@ -16,7 +16,7 @@ constexpr int kSampleRowCands = 4096;           // candidates of a row the finis
 // need-th largest of its threads' maxima: with the values in random order, as many as it takes to meet `need` different threads,
 // 256 ln(1 / (1 - x)) of them with x = need / 256, variance 256 (x / (1 - x) + ln(1 - x)). Admitted up to six standard deviations:
 // 96 at 128 256 logits, 84 at 151 936, 67 at 201 088, 54 at 262 144. Rows that overflow pay for the chunks and the general
-// passes (a step of 160 rows of 201 088 logits, top_k 80: 7296 us, against 7109 by the general passes alone; 1203 at top_k 64
+// passes (a step of 160 rows of 201 088 logits, top_k 80: 7296 us, against 6931 by the general passes alone; 1203 at top_k 64
 // from lists that fit).
 inline bool sample_candidates_fit(int n_vocab, int need) {
     if (need <= 0) return true;

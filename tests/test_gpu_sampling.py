@@ -182,3 +182,20 @@ def test_top_k_at_the_limits_of_the_candidate_lists(rb, oracle, models):
                     assert out.row(slot).token == want or margin < 1e-9
                     assert list(out.top(slot)[0]) == np.argsort(-l, kind="stable")[:3].tolist()
     assert launches[64] == launches[96] == launches[97] + 1 and launches[97] == launches[100] == launches[128]
+
+
+@pytest.mark.parametrize("vocab", [260, 8191, 8192, 8193, 16385])
+def test_rows_of_the_general_passes_match_the_restatement(rb, oracle, models, vocab):
+    """min_p and a nucleus over the whole vocabulary: the row is copied eight times 1024 logits at a time, then transformed."""
+    path = models(f"sampling_{vocab}", arch="llama", layers=1, d=256, heads=4, kv_heads=4, ff=256, vocab=vocab, dtype="q8_0", seed=9)
+    options = [dict(min_p=0.1), dict(min_p=0.3, temperature=1.5, logit_bias=[(vocab - 1, 4.0)]), dict(top_p=0.8), dict(top_k=129, top_p=0.5)]
+    with rb.Engine(str(path), rb.EngineConfig(n_ctx=256, n_seq_max=4, n_batch=64, n_ubatch=64)) as engine:
+        out = rb.StepOutput()
+        for draw in range(4):
+            params = [rb.SamplingParamsV2(seed=20 + i, **o) for i, o in enumerate(options)]
+            engine.step([rb.StepRow(i, i, [5 + draw], draw, True, sp, 0, True) for i, sp in enumerate(params)], out)
+            for i, sp in enumerate(params):
+                logits, o = engine.last_logits(i), out.row(i)
+                want, margin = oracle.sample_philox(_transformed(logits, sp), sp.temperature, sp.top_p, sp.seed, draw)
+                assert o.token == want or margin < 1e-9
+                assert o.logprob == pytest.approx(float(oracle.token_logprob(logits, o.token)), abs=2e-6)
