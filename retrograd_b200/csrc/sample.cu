@@ -384,7 +384,7 @@ struct RowShared {
     int32_t by_id[kListMax];        // kept entries in id order
     int32_t offset[kThreads];       // first candidate of each chunk
     double total, rtotal, mass, prefix;
-    float rmax, tmax;
+    float rmax, tmax, token_logit;
     int32_t rarg, targ, n_keep, token, chunk, n_list;
 };
 
@@ -666,17 +666,20 @@ __device__ bool row_from_chunks(Shared & sh, RowShared & rs, const float * __res
         }
     }
     if (token < 0 || token >= V) token = 0;      // a row of NaNs has no arg-max: stay inside the row
+    const bool want_logprob = v2 && (d.flags & kFlagWantLogprob);
+    if (want_logprob) {
+        // the whole block looks for the token's edit: a long history has as many edits as distinct tokens
+        if (tid == 0) rs.token_logit = raw[token];
+        __syncthreads();
+        for (uint32_t e = d.edit_begin + tid; e < d.edit_end; e += kThreads)
+            if (edits[e].id == token) rs.token_logit = edited(raw[token], edits[e]);
+        __syncthreads();
+    }
     if (tid == 0) {
         SampleOut o;
         o.token = token;
         o.logprob = (float)((double)raw[token] - (double)rmax - rlog);
-        o.sampled_logprob = 0.f;
-        if (v2 && (d.flags & kFlagWantLogprob)) {
-            float lt = raw[token];
-            for (uint32_t e = d.edit_begin; e < d.edit_end; ++e)
-                if (edits[e].id == token) lt = edited(lt, edits[e]);
-            o.sampled_logprob = (float)log(exp(((double)lt - (double)tmax) * inv_t) / kept);
-        }
+        o.sampled_logprob = want_logprob ? (float)log(exp(((double)rs.token_logit - (double)tmax) * inv_t) / kept) : 0.f;
         o.n_top = n_top;
         *out = o;
     }

@@ -199,3 +199,50 @@ def test_rows_of_the_general_passes_match_the_restatement(rb, oracle, models, vo
                 want, margin = oracle.sample_philox(_transformed(logits, sp), sp.temperature, sp.top_p, sp.seed, draw)
                 assert o.token == want or margin < 1e-9
                 assert o.logprob == pytest.approx(float(oracle.token_logprob(logits, o.token)), abs=2e-6)
+
+
+def _penalised(logits, sp, history):
+    """Biases summed per id, then the penalties of the window, each step rounded to f32 as the kernel does."""
+    l = logits.copy()
+    edits = {}
+    for token, bias in sp.logit_bias:
+        edits.setdefault(token, [np.float32(0), 0])[0] += np.float32(bias)
+    window = history[-sp.penalty_window :] if sp.penalty_window else history
+    for token in window:
+        edits.setdefault(token, [np.float32(0), 0])[1] += 1
+    for token, (bias, count) in edits.items():
+        t = np.float32(l[token] + bias)
+        if count:
+            rp = np.float32(sp.repeat_penalty)
+            t = np.float32(t * rp) if t <= 0 else np.float32(t / rp)
+            t -= np.float32(np.float32(count) * np.float32(sp.frequency_penalty)) + np.float32(sp.presence_penalty)
+        l[token] = t
+    return l
+
+
+def test_penalties_over_a_history_and_a_full_bias_list(rb, oracle, models):
+    """Rows whose edits grow with their history, and one with 4096 biases (the largest list that is accepted), served from the
+    chunks: token, sampled log-probability and top list against the restatement."""
+    path = models("sampling_20000", arch="llama", layers=1, d=256, heads=4, kv_heads=4, ff=256, vocab=20000, dtype="q8_0", seed=6)
+    bias = [(int(i), float(b)) for i, b in zip(np.random.default_rng(0).permutation(20000)[:4096], np.random.default_rng(1).normal(0, 2, 4096))]
+    options = [dict(top_k=3, repeat_penalty=1.3), dict(top_k=30, frequency_penalty=0.7, presence_penalty=0.4), dict(repeat_penalty=0.7, penalty_window=4),
+               dict(top_k=2, logit_bias=bias, repeat_penalty=1.1), dict(temperature=0.9, logit_bias=bias)]
+    histories = [[] for _ in options]
+    with rb.Engine(str(path), rb.EngineConfig(n_ctx=1024, n_seq_max=8, n_batch=64, n_ubatch=64)) as engine:
+        out = rb.StepOutput()
+        for draw in range(24):
+            params = [rb.SamplingParamsV2(seed=70 + i, **o) for i, o in enumerate(options)]
+            engine.step([rb.StepRow(i, i, [5 + draw % 3], draw, True, sp, 3, True) for i, sp in enumerate(params)], out)
+            for i, sp in enumerate(params):
+                logits, o = engine.last_logits(i), out.row(i)
+                l = _penalised(logits, sp, histories[i])
+                if sp.top_k:
+                    l[np.argsort(-l, kind="stable")[sp.top_k :]] = -np.inf
+                want, margin = oracle.sample_philox(l, sp.temperature, 1.0, sp.seed, draw)
+                assert o.token == want or margin < 1e-9
+                p = np.exp((l.astype(np.float64) - l.max()) / np.float32(sp.temperature))
+                assert o.sampled_logprob == pytest.approx(np.log(p[o.token] / p.sum()), abs=1e-5)
+                assert o.logprob == pytest.approx(float(oracle.token_logprob(logits, o.token)), abs=2e-6)
+                assert list(out.top(i)[0]) == np.lexsort((np.arange(l.size), -l))[:3].tolist()
+                histories[i].append(o.token)
+    assert len(set(histories[0])) > 3
