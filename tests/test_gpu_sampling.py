@@ -246,3 +246,23 @@ def test_penalties_over_a_history_and_a_full_bias_list(rb, oracle, models):
                 assert list(out.top(i)[0]) == np.lexsort((np.arange(l.size), -l))[:3].tolist()
                 histories[i].append(o.token)
     assert len(set(histories[0])) > 3
+
+
+def test_sampled_row_counts_that_rise_and_fall(rb, models):
+    """The output projection's activations keep the layout of the most rows so far: 24 rows after 40 give the logits of 24 rows in
+    an engine of their own, bit for bit, on the tensor-core path of either weight type."""
+    for dtype in ("q4_k", "q8_0"):
+        path = models(f"sampling_rows_{dtype}", arch="llama", layers=1, d=512, heads=4, kv_heads=4, ff=512, vocab=1000, dtype=dtype, seed=8)
+
+        def logits(counts):
+            with rb.Engine(str(path), rb.EngineConfig(n_ctx=4096, n_seq_max=64, n_batch=256, n_ubatch=256)) as engine:
+                out = rb.StepOutput()
+                for n in counts:
+                    for i in range(n):
+                        engine.seq_rm(i)
+                    engine.step([rb.StepRow(100 * n + i, i, [5 + i, 7], 0, True, rb.SamplingParamsV2.greedy()) for i in range(n)], out)
+                return np.stack([engine.last_logits(i) for i in range(counts[-1])])
+
+        want = logits([24])
+        assert np.isfinite(want).all()
+        assert np.array_equal(logits([3, 40, 1, 24]), want) and np.array_equal(logits([24, 17, 24]), want)
