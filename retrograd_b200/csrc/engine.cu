@@ -617,12 +617,13 @@ bool Engine::linear(const WeightView & w, const float * x, int ldx, int T, float
     } else if (xs && T > mma_min_tokens && gemm_q4k_exact_supported(w, *xs)) {
         launch_gemm_q4k_exact(w, *xs, T, y, ldy, bias, residual, ldr, stream);
     } else if (xs && T > mma_min_tokens && q8_tc5_ && gemm_q8_0_tc5_supported(w, *xs)) {
-        const size_t need = gemm_q8_0_tc5_scratch_floats(w.n_out, w.n_in, T, n_sm_);
+        const FinishTail * fused = tail && fused_finish_ && finish_tail_supported(*tail, (int)w.n_out, y, ldy, bias, residual, ldr) ? tail : nullptr;
+        const size_t need = gemm_q8_0_tc5_scratch_floats(w.n_out, w.n_in, T, n_sm_, fused != nullptr);
         if (need) stream_scratch_.ensure(need);
-        tail_done = need && tail && fused_finish_ && finish_tail_supported(*tail, (int)w.n_out, y, ldy, bias, residual, ldr);
-        launch_gemm_q8_0_tc5(w, *xs, T, y, ldy, bias, residual, ldr, device_error_.ptr, stream_scratch_.ptr, n_sm_, stream, tail_done ? tail : nullptr);
+        tail_done = need && fused;
+        launch_gemm_q8_0_tc5(w, *xs, T, y, ldy, bias, residual, ldr, device_error_.ptr, stream_scratch_.ptr, n_sm_, stream, fused);
         if (need) ++last_launches;
-} else if (xs && T > mma_min_tokens && gemm_q8_0_exact_supported(w, *xs)) {
+    } else if (xs && T > mma_min_tokens && gemm_q8_0_exact_supported(w, *xs)) {
         launch_gemm_q8_0_exact(w, *xs, T, y, ldy, bias, residual, ldr, stream);
     } else {
         launch_gemm_rows(w, x, ldx, T, y, ldy, bias, residual, ldr, stream);

@@ -30,6 +30,7 @@
 #include "blocks.hpp"
 #include "mma_common.cuh"
 #include "tc5_common.cuh"
+#include "q8_0_tc5_plan.hpp"
 
 namespace rb200 {
 
@@ -37,7 +38,6 @@ namespace {
 
 constexpr int BM = 128;
 constexpr int TMEM_COLS = 512;
-constexpr int kMaxSplits = 8, kMinSplitStages = 8;
 
 // A producer warp reads the 32 x 68 bytes of its rows' stage segments as 544 consecutive-per-row words - lane after
 // lane along a row, so a load instruction touches two or three rows instead of 32 - and hands every lane its own
@@ -315,44 +315,12 @@ void launch_form(const WeightView & w, const SplitAct & x, int n_tokens, float *
     else launch_one<BN, false, false>(w, x, n_tokens, y, ldy, bias, nullptr, 0, error_flag, 1, nullptr, stream);
 }
 
-struct Plan {
-    bool wide;
-    int splits;
-};
-
-// The form and the number of splits with the shortest estimated time, in cycles, for whole waves of one CTA per SM.
-// 256-token tiles halve the decode work per product (measured per 64-column stage: about 1800 cycles at N = 256, where the
-// twelve MMAs take 1536, and 1300 at N = 128, where the producers set the pace; narrower MMAs do not help the producers). A
-// split costs the write and the read of its partial results (about 2000 bytes per cycle) and the finish kernel a launch;
-// every wave pays for its CTAs' beginning and end. Unsplit, 4096 x 14 336 took 153 us and 4096 x 4096 50 us from 24 tokens to
-// 512 (32 row tiles on 148 SMs); with the splits a step of 320 rows over eight layers of the 8B shape went from 8437 to 7879 us,
-// two steps of 24 rows over four layers of the 20B-class mixture of experts from 4725 to 4354 us.
-Plan plan_of(uint32_t n_out, uint32_t n_in, int n_tokens, int n_sm) {
+Q8Tc5Plan plan_of(uint32_t n_out, uint32_t n_in, int n_tokens, int n_sm, bool tail) {
     static const int forced = [] {          // RB200_Q8_TC5_TILE=128|256 pins the form (measurements)
         const char * env = std::getenv("RB200_Q8_TC5_TILE");
         return env ? std::atoi(env) : 0;
     }();
-    const int n_it = (int)n_in / 64, row_tiles = (int)((n_out + BM - 1) / BM);
-    Plan best{false, 1};
-    long long best_cycles = -1;
-    for (int wide = 0; wide < 2; ++wide) {
-        if (wide && (n_tokens <= 128 || forced == 128)) continue;
-        if (!wide && n_tokens > 128 && forced == 256) continue;
-        const long long tiles = (long long)row_tiles * ((n_tokens + (wide ? 255 : 127)) / (wide ? 256 : 128));
-        for (int splits = 1; splits <= kMaxSplits && (splits == 1 || n_it / splits >= kMinSplitStages); ++splits) {
-            const int per_split = (n_it + splits - 1) / splits;
-            if ((n_it + per_split - 1) / per_split != splits) continue;      // an empty last range
-            if (splits > 1 && tiles * splits > n_sm) break;                  // a split that does not fit one wave gains too little for its traffic
-            const long long waves = (tiles * splits + n_sm - 1) / n_sm;
-            long long cycles = waves * ((long long)per_split * (wide ? 1800 : 1300) + 6000);
-            if (splits > 1) cycles += 6000 + (long long)splits * n_tokens * n_out * 8 / 2000;
-            if (best_cycles < 0 || cycles < best_cycles) {
-                best_cycles = cycles;
-                best = Plan{wide != 0, splits};
-            }
-        }
-    }
-    return best;
+    return q8_0_tc5_plan(n_out, n_in, n_tokens, n_sm, tail, forced);
 }
 
 } // namespace
@@ -374,15 +342,15 @@ bool gemm_q8_0_tc5_supported(const WeightView & w, const SplitAct & x) {
            x.ld == (int)w.n_in && x.has_maps;
 }
 
-size_t gemm_q8_0_tc5_scratch_floats(uint32_t n_out, uint32_t n_in, int n_tokens, int n_sm) {
-    const int splits = plan_of(n_out, n_in, n_tokens, n_sm).splits;
+size_t gemm_q8_0_tc5_scratch_floats(uint32_t n_out, uint32_t n_in, int n_tokens, int n_sm, bool tail) {
+    const int splits = plan_of(n_out, n_in, n_tokens, n_sm, tail).splits;
     return splits > 1 ? (size_t)splits * n_tokens * n_out : 0;
 }
 
 void launch_gemm_q8_0_tc5(const WeightView & w, const SplitAct & x, int n_tokens, float * y, int ldy, const float * bias, const float * residual,
                           int ldr, int * error_flag, float * scratch, int n_sm, cudaStream_t stream, const FinishTail * tail) {
     if (n_tokens <= 0) return;
-    const Plan plan = plan_of(w.n_out, w.n_in, n_tokens, n_sm);
+    const Q8Tc5Plan plan = plan_of(w.n_out, w.n_in, n_tokens, n_sm, tail != nullptr);
     if (plan.wide) launch_form<256>(w, x, n_tokens, y, ldy, bias, residual, ldr, error_flag, plan.splits, scratch, stream);
     else launch_form<128>(w, x, n_tokens, y, ldy, bias, residual, ldr, error_flag, plan.splits, scratch, stream);
     if (plan.splits > 1) launch_gemm_stream_finish(scratch, plan.splits, (int)w.n_out, n_tokens, n_tokens, y, ldy, bias, residual, ldr, stream, tail);

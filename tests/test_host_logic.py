@@ -177,6 +177,27 @@ def test_sampling_rows_are_admitted_to_candidate_lists_that_hold_them(tmp_path):
     assert out.returncode == 0, out.stdout + out.stderr
 
 
+def _q8_0_plans(tmp_path, shapes):
+    """(tile height, splits, stages of the last range, stages of a range) of the Q8_0 tcgen05 GEMM for each (rows, columns, tokens, tail)."""
+    exe = tmp_path / "q8_0_tc5_plan"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-o", str(exe), str(ROOT / "tests" / "cpp" / "q8_0_tc5_plan.cpp")], check=True)
+    out = subprocess.run([str(exe)] + [str(v) for shape in shapes for v in shape], capture_output=True, text=True, check=True).stdout
+    return [tuple(int(v) for v in line.split()) for line in out.splitlines()]
+
+
+def test_q8_0_reduction_is_split_only_where_that_was_measured_faster(tmp_path):
+    """Sizes of the 8B and the 20B-class projections around the border: tile height and splits of the fastest form measured."""
+    fastest = {(4096, 4096, 17, 0): (128, 4), (4096, 4096, 128, 0): (128, 4), (4096, 4096, 200, 0): (256, 4), (4096, 4096, 300, 0): (128, 1),
+               (4096, 4096, 384, 0): (128, 1), (4096, 4096, 512, 0): (128, 1), (4096, 4096, 1024, 0): (256, 1), (4096, 2880, 200, 0): (256, 4),
+               (4096, 2880, 320, 0): (128, 1), (4096, 14336, 200, 0): (256, 4), (4096, 14336, 512, 0): (256, 2), (4096, 14336, 768, 0): (256, 1),
+               (6144, 4096, 128, 0): (128, 3), (6144, 4096, 300, 0): (128, 1), (2880, 4096, 24, 0): (128, 6), (2880, 4096, 640, 0): (128, 1),
+               (2880, 4096, 768, 0): (128, 1), (2048, 2048, 640, 0): (128, 1), (8192, 1024, 64, 0): (128, 1), (1024, 4096, 24, 0): (128, 8),
+               (28672, 4096, 1781, 0): (256, 1), (201088, 2880, 24, 0): (128, 1),
+               # with the RMS norm behind it the finish kernel takes its place
+               (4096, 4096, 320, 1): (256, 2), (4096, 4096, 437, 1): (256, 2), (2880, 4096, 640, 1): (256, 2), (4096, 4096, 1024, 1): (256, 1)}
+    assert [p[:2] for p in _q8_0_plans(tmp_path, fastest)] == list(fastest.values())
+
+
 def test_mxfp4_expert_blocks_recode_exactly_as_q8_0(rb, oracle):
     """The engine holds MXFP4 expert banks as Q8_0 for the tensor cores: the doubled E2M1 value as the int8,
     half the E8M0 scale as the f16 d. Every value must decode to the same f32; a scale an f16 cannot hold
