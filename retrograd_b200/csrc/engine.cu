@@ -620,8 +620,8 @@ bool Engine::linear(const WeightView & w, const float * x, int ldx, int T, float
         const FinishTail * fused = tail && fused_finish_ && finish_tail_supported(*tail, (int)w.n_out, y, ldy, bias, residual, ldr) ? tail : nullptr;
         const size_t need = gemm_q8_0_tc5_scratch_floats(w.n_out, w.n_in, T, n_sm_, fused != nullptr);
         if (need) stream_scratch_.ensure(need);
-        tail_done = need && fused;
-        launch_gemm_q8_0_tc5(w, *xs, T, y, ldy, bias, residual, ldr, device_error_.ptr, stream_scratch_.ptr, n_sm_, stream, fused);
+        tail_done = launch_gemm_q8_0_tc5(w, *xs, T, y, ldy, bias, residual, ldr, device_error_.ptr, stream_scratch_.ptr, stream_scratch_.count, n_sm_,
+                                         stream, fused);
         if (need) ++last_launches;
     } else if (xs && T > mma_min_tokens && gemm_q8_0_exact_supported(w, *xs)) {
         launch_gemm_q8_0_exact(w, *xs, T, y, ldy, bias, residual, ldr, stream);

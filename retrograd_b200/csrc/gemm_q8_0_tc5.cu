@@ -347,13 +347,16 @@ size_t gemm_q8_0_tc5_scratch_floats(uint32_t n_out, uint32_t n_in, int n_tokens,
     return splits > 1 ? (size_t)splits * n_tokens * n_out : 0;
 }
 
-void launch_gemm_q8_0_tc5(const WeightView & w, const SplitAct & x, int n_tokens, float * y, int ldy, const float * bias, const float * residual,
-                          int ldr, int * error_flag, float * scratch, int n_sm, cudaStream_t stream, const FinishTail * tail) {
-    if (n_tokens <= 0) return;
-    const Q8Tc5Plan plan = plan_of(w.n_out, w.n_in, n_tokens, n_sm, tail != nullptr);
+bool launch_gemm_q8_0_tc5(const WeightView & w, const SplitAct & x, int n_tokens, float * y, int ldy, const float * bias, const float * residual,
+                          int ldr, int * error_flag, float * scratch, size_t scratch_floats, int n_sm, cudaStream_t stream, const FinishTail * tail) {
+    if (n_tokens <= 0) return false;
+    Q8Tc5Plan plan = plan_of(w.n_out, w.n_in, n_tokens, n_sm, tail != nullptr);
+    if (plan.splits > 1 && (!scratch || (size_t)plan.splits * n_tokens * w.n_out > scratch_floats)) plan.splits = 1;
     if (plan.wide) launch_form<256>(w, x, n_tokens, y, ldy, bias, residual, ldr, error_flag, plan.splits, scratch, stream);
     else launch_form<128>(w, x, n_tokens, y, ldy, bias, residual, ldr, error_flag, plan.splits, scratch, stream);
-    if (plan.splits > 1) launch_gemm_stream_finish(scratch, plan.splits, (int)w.n_out, n_tokens, n_tokens, y, ldy, bias, residual, ldr, stream, tail);
+    if (plan.splits == 1) return false;
+    launch_gemm_stream_finish(scratch, plan.splits, (int)w.n_out, n_tokens, n_tokens, y, ldy, bias, residual, ldr, stream, tail);
+    return tail != nullptr;
 }
 
 } // namespace rb200

@@ -361,11 +361,12 @@ void launch_gemm_q8_0_stream(const WeightView & w, const SplitAct & x, int n_tok
 bool q8_0_products_fit_f16(const uint8_t * blocks, size_t n_blocks);
 bool gemm_q8_0_tc5_supported(const WeightView & w, const SplitAct & x);
 // Where the output tiles leave SMs idle the reduction is cut into splits (grid.z) whose partial results, in `scratch`
-// (gemm_q8_0_tc5_scratch_floats() floats, 0 without splits), a finish kernel adds in order; the tail is done only then.
-// `tail`: whether the launch will be given one (the plan depends on it).
+// (gemm_q8_0_tc5_scratch_floats() floats, 0 without splits), a finish kernel adds in order. With less scratch the reduction
+// stays whole. `tail`: whether the launch will be given one (the plan depends on it). Returns whether the tail was done: only
+// the finish kernel does it.
 size_t gemm_q8_0_tc5_scratch_floats(uint32_t n_out, uint32_t n_in, int n_tokens, int n_sm, bool tail);
-void launch_gemm_q8_0_tc5(const WeightView & w, const SplitAct & x, int n_tokens, float * y, int ldy, const float * bias, const float * residual,
-                          int ldr, int * error_flag, float * scratch, int n_sm, cudaStream_t stream, const FinishTail * tail = nullptr);
+bool launch_gemm_q8_0_tc5(const WeightView & w, const SplitAct & x, int n_tokens, float * y, int ldy, const float * bias, const float * residual,
+                          int ldr, int * error_flag, float * scratch, size_t scratch_floats, int n_sm, cudaStream_t stream, const FinishTail * tail = nullptr);
 // Exact tensor-core Q8_0 GEMM (mma.sync) for more than 8 tokens; reads the GGUF-layout rows.
 bool gemm_q8_0_exact_supported(const WeightView & w, const SplitAct & x);
 void launch_gemm_q8_0_exact(const WeightView & w, const SplitAct & x, int n_tokens, float * y, int ldy, const float * bias,

@@ -12,7 +12,8 @@ using namespace rb200;
 extern "C" {
 
 // y[t][o] = sum_k deq(w)[o][k] x[t][k]. `path`: 0 = what the engine would pick, 1 = f32 row kernel,
-// 3 = exact tensor-core kernel (mma.sync), 4 = exact tcgen05 kernel, 5 = exact weight-streaming kernel (at most 8 tokens). The kernel runs `iters`
+// 3 = exact tensor-core kernel (mma.sync), 4 = exact tcgen05 kernel, 5 = exact weight-streaming kernel (at most 8 tokens), 6 = the tcgen05 kernel
+// without scratch for splits of the reduction, which then stays whole. The kernel runs `iters`
 // times; *out_ms receives the mean device time per launch (CUDA events on the launching stream).
 int retro_b200_op_gemm(uint32_t ggml_type, const uint8_t * w, uint32_t n_out, uint32_t n_in, const float * x, uint32_t n_tokens, float * y,
                        int path, uint32_t iters, float * out_ms) {
@@ -43,7 +44,7 @@ int retro_b200_op_gemm(uint32_t ggml_type, const uint8_t * w, uint32_t n_out, ui
         wv.n_out = n_out;
         wv.row_bytes = (uint32_t)rb;
         DeviceBuffer<uint8_t> dtiled;
-        if (ggml_type == GGML_Q4_K && n_in % 256 == 0 && (path == 4 || path == 5 || path == 0)) {
+        if (ggml_type == GGML_Q4_K && n_in % 256 == 0 && (path == 4 || path == 5 || path == 6 || path == 0)) {
             dtiled.ensure(q4k_tiled_bytes(n_out, n_in));
             launch_q4k_retile(dw.ptr, n_out, n_in, (uint32_t)rb, dtiled.ptr, stream);
             wv.tiled = dtiled.ptr;
@@ -57,7 +58,8 @@ int retro_b200_op_gemm(uint32_t ggml_type, const uint8_t * w, uint32_t n_out, ui
         if (ggml_type == GGML_Q8_0 && n_in % 64 == 0) wv.tc5_exact = q8_0_products_fit_f16(w, (size_t)n_out * (n_in / 32));
         const bool have_split = xs.get() != nullptr;
         if (have_split) launch_split_prep(dx.ptr, (int)n_in, (int)n_in, (int)n_tokens, xs.view, stream);
-        int chosen = path;
+        const bool with_scratch = path != 6;
+        int chosen = path == 6 ? 4 : path;
         if (chosen == 0) chosen = have_split && n_tokens > 64 && gemm_q4k_tc5_supported(wv, xs.view) ? 4 : have_split && n_tokens > 8 && gemm_q4k_exact_supported(wv, xs.view) ? 3 : 1;
         DeviceBuffer<float> tc5_scratch;
         DeviceBuffer<int> flag;
@@ -78,11 +80,11 @@ int retro_b200_op_gemm(uint32_t ggml_type, const uint8_t * w, uint32_t n_out, ui
             }
             stream_scratch.ensure(gemm_q4k_stream_scratch_floats(n_out, n_in));
         }
-        if (chosen == 4 && ggml_type == GGML_Q4_K) {
+        if (chosen == 4 && with_scratch && ggml_type == GGML_Q4_K) {
             const size_t need = gemm_q4k_tc5_scratch_floats(wv.n_out, wv.n_in, (int)n_tokens, n_sm);
             if (need) tc5_scratch.ensure(need);
         }
-        if (chosen == 4 && ggml_type == GGML_Q8_0) {
+        if (chosen == 4 && with_scratch && ggml_type == GGML_Q8_0) {
             const size_t need = gemm_q8_0_tc5_scratch_floats(wv.n_out, wv.n_in, (int)n_tokens, n_sm, false);
             if (need) tc5_scratch.ensure(need);
         }
@@ -99,7 +101,7 @@ int retro_b200_op_gemm(uint32_t ggml_type, const uint8_t * w, uint32_t n_out, ui
         auto run = [&]() {
             if (chosen == 5 && ggml_type == GGML_Q8_0) launch_gemm_q8_0_stream(wv, xs.view, (int)n_tokens, dy.ptr, (int)n_out, nullptr, nullptr, 0, stream_scratch.ptr, n_sm, flag.ptr, stream);
             else if (chosen == 5) launch_gemm_q4k_stream(wv, xs.view, (int)n_tokens, dy.ptr, (int)n_out, nullptr, nullptr, 0, stream_scratch.ptr, n_sm, flag.ptr, stream);
-            else if (chosen == 4 && ggml_type == GGML_Q8_0) launch_gemm_q8_0_tc5(wv, xs.view, (int)n_tokens, dy.ptr, (int)n_out, nullptr, nullptr, 0, flag.ptr, tc5_scratch.ptr, n_sm, stream);
+            else if (chosen == 4 && ggml_type == GGML_Q8_0) launch_gemm_q8_0_tc5(wv, xs.view, (int)n_tokens, dy.ptr, (int)n_out, nullptr, nullptr, 0, flag.ptr, tc5_scratch.ptr, tc5_scratch.count, n_sm, stream);
             else if (chosen == 4) launch_gemm_q4k_tc5(wv, xs.view, (int)n_tokens, dy.ptr, (int)n_out, nullptr, nullptr, 0, flag.ptr, tc5_scratch.ptr, tc5_scratch.count, n_sm, stream);
             else if (chosen == 3 && ggml_type == GGML_Q8_0) launch_gemm_q8_0_exact(wv, xs.view, (int)n_tokens, dy.ptr, (int)n_out, nullptr, nullptr, 0, stream);
             else if (chosen == 3) launch_gemm_q4k_exact(wv, xs.view, (int)n_tokens, dy.ptr, (int)n_out, nullptr, nullptr, 0, stream);

@@ -179,3 +179,23 @@ def test_q8_0_tcgen05_splits_of_the_reduction(rb, oracle, n_out, n_in, T):
     got, _ = rb.op_gemm(8, raw, n_out, n_in, x, path=4)
     scale = np.abs(wd).max(axis=1) * np.abs(x).max() * np.sqrt(n_in)
     assert float((np.abs(got - want) / scale[None, :]).max()) < 2e-5
+
+
+@pytest.mark.parametrize("n_out,n_in,T", [(512, 2048, 130), (256, 4096, 300), (1000, 4096, 40), (300, 14336, 33)])
+def test_q8_0_tcgen05_keeps_the_reduction_whole_without_scratch(rb, oracle, n_out, n_in, T):
+    """The same kernel given no room for partial results (each of these shapes would be split): one accumulator over up to 14 336
+    columns. It rounds towards zero inside the tensor core, so the error grows with the row length: at most 224 stages of
+    64 columns at 2^-23 of the largest partial sum each, 3e-5 of it."""
+    rng = np.random.default_rng(23 * n_out + T)
+    w = rng.normal(0, 0.02, (n_out, n_in)).astype(np.float32)
+    raw = np.frombuffer(b"".join(rb.quantize_row(8, w[r]) for r in range(n_out)), dtype=np.uint8)
+    x = rng.normal(0, 1.5, (T, n_in)).astype(np.float32)
+    wd = oracle.dequantize_row(oracle.T_Q8_0, raw, n_out * n_in).reshape(n_out, n_in).astype(np.float64)
+    want = x.astype(np.float64) @ wd.T
+    scale = np.abs(wd).max(axis=1) * np.abs(x).max() * np.sqrt(n_in)
+    whole, _ = rb.op_gemm(8, raw, n_out, n_in, x, path=6)
+    split, _ = rb.op_gemm(8, raw, n_out, n_in, x, path=4)
+    err_whole, err_split = (float((np.abs(y - want) / scale[None, :]).max()) for y in (whole, split))
+    print(f"q8_0 tcgen05 {n_out}x{n_in} T={T}: scaled err {err_whole:.2e} whole, {err_split:.2e} split")
+    assert err_whole < (2e-5 if n_in <= 4096 else 3e-5) and err_split < 2e-5
+    assert not np.array_equal(whole, split)
