@@ -419,6 +419,28 @@ def test_finish_kernel_tails_equal_the_separate_kernels(rb, models, monkeypatch,
         assert t0 == t1 and l0 == l1 and np.array_equal(x0, x1)
 
 
+@pytest.mark.parametrize("arch,bias", [("llama", 0), ("qwen2", 1)])
+def test_split_reductions_with_tails_equal_the_separate_kernels(rb, models, monkeypatch, arch, bias):
+    """Q8_0 steps of more than 16 tokens whose projections (3072, 2048, 4096 and 2048 rows of 2048 columns) are all split, with
+    tails or without: the finish kernels' norm, RoPE with store, and SwiGLU, bit for bit those of the separate kernels."""
+    path = models(f"tails_split_{arch}", arch=arch, layers=2, d=2048, heads=32, kv_heads=8, ff=2048, vocab=512, dtype="q8_0", seed=44, bias=bias)
+
+    def run(fused: bool):
+        monkeypatch.setenv("RB200_FUSED_FINISH", "1" if fused else "0")
+        trace, pos = [], [0, 0, 0]
+        with rb.Engine(str(path), rb.EngineConfig(n_ctx=2048, n_seq_max=4, n_batch=256, n_ubatch=256)) as engine:
+            out = rb.StepOutput()
+            for step, lengths in enumerate([(8, 8, 8), (70, 70, 60), (24, 23, 23)]):
+                rows = [rb.StepRow(i, i, _prompt(500 + 10 * step + i, n, 512), pos[i], True, rb.SamplingParamsV2.greedy(), 0, True) for i, n in enumerate(lengths)]
+                engine.step(rows, out)
+                pos = [p + n for p, n in zip(pos, lengths)]
+                trace.append((engine.last_step_stats()[1], np.stack([engine.last_logits(i) for i in range(3)])))
+        return trace
+
+    for (n0, separate), (n1, fused) in zip(run(False), run(True)):
+        assert n1 < n0 and np.array_equal(separate, fused)
+
+
 def _greedy_v1(n_new, seed=0):
     # the serving layer's spelling of greedy for v1 rows: a nucleus that holds one token
     return dict(temperature=1e-4, top_p=1e-6, max_new_tokens=n_new, seed=seed)

@@ -166,10 +166,18 @@ def test_mxfp4_grouped_tcgen05_gemm_against_float64(rb, oracle, n_expert, n_out,
     assert worst < 2e-5         # one tensor-core accumulator over the whole row, as for Q8_0 above
 
 
-@pytest.mark.parametrize("n_out,n_in,T", [(128, 1024, 17), (200, 1216, 33), (256, 4096, 128), (384, 2880, 129), (2048, 1088, 300)])
+# (rows, columns, tokens): token tile, splits, 64-column stages of the last range, of the others. A host test compares them with
+# the kernel's plan.
+Q8_SPLITS = {
+    (128, 1024, 17): (128, 2, 8, 8), (200, 1216, 33): (128, 2, 9, 10), (256, 4096, 128): (128, 8, 8, 8), (384, 2880, 129): (128, 5, 9, 9),
+    (200, 4160, 257): (128, 8, 2, 9), (2176, 2048, 257): (256, 4, 8, 8), (2944, 8192, 300): (256, 3, 42, 43), (1152, 4096, 700): (256, 5, 12, 13),
+}
+
+
+@pytest.mark.parametrize("n_out,n_in,T", Q8_SPLITS)
 def test_q8_0_tcgen05_splits_of_the_reduction(rb, oracle, n_out, n_in, T):
-    """Few output tiles: the reduction is cut into ranges of stages (16 to 64 of them here, a short last range in the second,
-    fourth and fifth shape), in both tile forms; bounds as for the whole reduction."""
+    """Few output tiles: the reduction is cut into two to eight ranges of stages, even ones and ones with a short last range, in
+    both tile forms; bounds as for the whole reduction."""
     rng = np.random.default_rng(n_out + n_in + T)
     w = rng.normal(0, 0.02, (n_out, n_in)).astype(np.float32)
     raw = np.frombuffer(b"".join(rb.quantize_row(8, w[r]) for r in range(n_out)), dtype=np.uint8)

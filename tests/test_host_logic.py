@@ -198,6 +198,18 @@ def test_q8_0_reduction_is_split_only_where_that_was_measured_faster(tmp_path):
     assert [p[:2] for p in _q8_0_plans(tmp_path, fastest)] == list(fastest.values())
 
 
+def test_the_split_shapes_of_the_kernel_test_are_split_as_it_says(tmp_path):
+    from test_gpu_ops import Q8_SPLITS
+
+    assert _q8_0_plans(tmp_path, [(*shape, 0) for shape in Q8_SPLITS]) == list(Q8_SPLITS.values())
+    # the projections of the engine test of the tails, whether or not a tail is given
+    shapes = [(n_out, 2048, tokens) for n_out in (2048, 3072, 4096) for tokens in (24, 70, 200)]
+    plans = _q8_0_plans(tmp_path, [(*shape, tail) for shape in shapes for tail in (0, 1)])
+    assert plans[::2] == plans[1::2] and all(p[1] > 1 for p in plans)
+    # and these are whole: the long reductions of the production shapes
+    assert {p[1] for p in _q8_0_plans(tmp_path, [(28672, 4096, 60, 1), (28672, 4096, 1781, 1), (128256, 4096, 30, 0), (6144, 4096, 320, 1)])} == {1}
+
+
 def test_mxfp4_expert_blocks_recode_exactly_as_q8_0(rb, oracle):
     """The engine holds MXFP4 expert banks as Q8_0 for the tensor cores: the doubled E2M1 value as the int8,
     half the E8M0 scale as the f16 d. Every value must decode to the same f32; a scale an f16 cannot hold
