@@ -16,7 +16,7 @@
 //              row p and stores them into lane p of the stage's A slot in TENSOR MEMORY (the MMA reads
 //              its A operand from there, so shared memory carries the activations only);
 //   20         walks the pipeline as a whole warp (uniform address arithmetic); one elected lane issues
-//              the MMAs (M 128, N the tile's height, K 16) and commits them to the stage's "empty" barrier, and per
+//              the MMAs (M 128, N the tile's tokens, K 16) and commits them to the stage's "empty" barrier, and per
 //              super-block to the accumulator's "full" barrier;
 //   21         fetches the two activation tiles (hi and lo) of a free slot with TMA, whose bytes
 //              complete on the stage's barrier;
@@ -143,6 +143,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_q4k_tc5_kernel(const uint8_t 
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int m0 = blockIdx.y * BM, t0 = blockIdx.x * tn;   // token tiles vary fastest: CTAs in flight share a weight tile in L2
+    // the last tile may have fewer tokens than its box is high: MMAs and epilogue take the columns it has, in whole MMA widths of 16
+    const int mma_n = min(tn, (T - t0 + 15) & ~15);
     // split-K: blockIdx.z owns super-blocks [sb0, sb0 + n_sb) of the row and writes a partial result
     const int n_sb_all = n_in / 256;
     const int sb0 = SPLIT ? blockIdx.z * sb_per_split : 0;
@@ -315,7 +317,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_q4k_tc5_kernel(const uint8_t 
             // uniform. (With a single thread inside a divergent branch the issuing thread - not the tensor
             // pipe - set the pace: 0.94 -> 0.81 ms on 28 672 x 4096 x 2048.) Descriptors are built once; a
             // stage costs an add per operand and the MMAs themselves.
-            const uint32_t idesc = tc5::instr_desc_f16(BM, tn);
+            const uint32_t idesc = tc5::instr_desc_f16(BM, mma_n);
             const uint64_t desc0 = tc5::smem_desc_sw128(smem_base);
             const uint32_t desc_lo0 = (uint32_t)desc0, desc_hi = (uint32_t)(desc0 >> 32);
             const uint32_t a_slot0 = tmem_base + TMEM_A;
@@ -378,7 +380,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_q4k_tc5_kernel(const uint8_t 
             const uint32_t t_main = t_lane + buf * 128;
 #pragma unroll
             for (int c = 0; c < 64; c += 8) {
-                if (colhalf * 64 + c < tn) {           // warp-uniform: columns that the MMAs do not write stay unread
+                if (colhalf * 64 + c < mma_n) {        // warp-uniform: columns that the MMAs do not write stay unread
                     float v[8];
                     tc5::tmem_ld8(t_main + c, v);
 #pragma unroll

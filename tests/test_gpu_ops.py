@@ -62,6 +62,18 @@ def test_q4k_tcgen05_token_tiles_of_every_height(rb, oracle, T):
     assert float(np.abs(got - want).max()) / float(np.abs(want).max()) < 4e-6
 
 
+@pytest.mark.parametrize("n_out,n_in,T", [(256, 512, 1025), (200, 768, 1041), (128, 1024, 1137), (384, 256, 1153)])
+def test_q4k_tcgen05_last_token_tile_of_its_own_width(rb, oracle, n_out, n_in, T):
+    """More than eight token tiles of 128, the last one with 1, 17, 113 and 1 tokens: its MMAs are 16, 32, 128 and 16 wide."""
+    rng = np.random.default_rng(T)
+    raw = _q4k_matrix(rb, rng, n_out, n_in)
+    x = rng.normal(0, 1.5, (T, n_in)).astype(np.float32)
+    w = oracle.dequantize_row(oracle.T_Q4_K, raw, n_out * n_in).reshape(n_out, n_in).astype(np.float64)
+    want = x.astype(np.float64) @ w.T
+    got, _ = rb.op_gemm(12, raw, n_out, n_in, x, path=4)
+    assert float(np.abs(got - want).max()) / float(np.abs(want).max()) < 4e-6
+
+
 @pytest.mark.parametrize("n_out,n_in,T", [(256, 512, 1), (384, 1024, 3), (200, 768, 8), (512, 2816, 5), (1040, 4096, 8), (128, 14336, 2)])
 def test_q4k_streaming_gemm_against_float64(rb, oracle, n_out, n_in, T):
     """The weight-streaming kernel for at most eight tokens: exact products, ragged row counts, and
