@@ -266,3 +266,46 @@ def test_sampled_row_counts_that_rise_and_fall(rb, models):
         want = logits([24])
         assert np.isfinite(want).all()
         assert np.array_equal(logits([3, 40, 1, 24]), want) and np.array_equal(logits([24, 17, 24]), want)
+
+
+def test_greedy_chunked_and_v1_rows_across_graph_replays(rb, oracle, models):
+    """Rows of every kind side by side, their numbers changing between steps of one shape while the steps are captured and
+    replayed: plain greedy rows beside rows of candidate lists (the chunk kernel's other form), untruncated draws, general rows."""
+    vocab = 20000
+    path = models(f"sampling_{vocab}", arch="llama", layers=1, d=256, heads=4, kv_heads=4, ff=256, vocab=vocab, dtype="q8_0", seed=6)
+    greedy, listed, plain, general = dict(top_k=1), dict(top_k=30, temperature=1.3), dict(), dict(min_p=0.1)
+    mixes = [[greedy] * 6, [greedy] * 4 + [listed] * 2, [listed] * 3 + [greedy] * 2 + [plain], [greedy, general, listed, greedy, plain, general]]
+    with rb.Engine(str(path), rb.EngineConfig(n_ctx=2048, n_seq_max=8, n_batch=64, n_ubatch=64)) as engine:
+        out = rb.StepOutput()
+        pos, draws = 0, [0] * 24
+        for mix in [0, 0, 0, 0, 1, 1, 1, 1, 0, 2, 2, 2, 1, 3, 3, 3, 2, 0, 3, 1]:
+            params = [rb.SamplingParamsV2(seed=90 + 6 * mix + i, **o) for i, o in enumerate(mixes[mix])]
+            engine.step([rb.StepRow(6 * mix + i, i, [5 + pos % 7 + i], pos, True, sp, 2, True) for i, sp in enumerate(params)], out)
+            for i, sp in enumerate(params):
+                logits = engine.last_logits(i)
+                l = _transformed(logits, sp)
+                want, margin = oracle.sample_philox(l, sp.temperature, 1.0, sp.seed, draws[6 * mix + i])
+                draws[6 * mix + i] += 1
+                assert out.row(i).token == want or margin < 1e-9, (pos, mix, i)
+                assert out.row(i).logprob == pytest.approx(float(oracle.token_logprob(logits, want)), abs=2e-6)
+                assert list(out.top(i)[0]) == np.lexsort((np.arange(vocab), -l))[:2].tolist()
+            pos += 1
+        assert engine.graph_stats()[0] >= 6
+
+
+@pytest.mark.parametrize("vocab", [260, 20000, 128256])
+def test_v1_rows_report_the_policy_before_the_draw(rb, oracle, models, vocab):
+    """v1 rows from the chunks: the draw at their temperature, token and top log-probabilities of the raw row."""
+    path = models(f"sampling_v1_{vocab}", arch="llama", layers=1, d=256, heads=4, kv_heads=4, ff=256, vocab=vocab, dtype="q8_0", seed=5)
+    with rb.Engine(str(path), rb.EngineConfig(n_ctx=256, n_seq_max=4, n_batch=64, n_ubatch=64)) as engine:
+        for draw in range(5):
+            params = [rb.SamplingParams(temperature=t, seed=10 + i) for i, t in enumerate((1.0, 0.6, 1.7))]
+            rows, ids, lps = engine.step_v1([rb.StepRow(i, i, [5 + draw], draw, True, sp, 6) for i, sp in enumerate(params)], 6)
+            for i, sp in enumerate(params):
+                logits = engine.last_logits(i)
+                want, margin = oracle.sample_philox(logits, sp.temperature, 1.0, sp.seed, draw)
+                assert rows[i].token == want or margin < 1e-9
+                assert rows[i].logprob == pytest.approx(float(oracle.token_logprob(logits, rows[i].token)), abs=2e-6)
+                want_ids, want_lps = oracle.top_token_logprobs(logits, 6)
+                assert ids[i].tolist() == want_ids.tolist()
+                np.testing.assert_allclose(lps[i], want_lps, atol=2e-6)
