@@ -42,7 +42,8 @@
 // once), and every other wait sleeps in hardware (try_wait with a time hint) instead of spinning.
 // Barrier arrivals are one per warp (after a warp-level synchronisation), not one per thread.
 // Every mbarrier wait is bounded: after about a second without progress the CTA raises an error
-// flag, drains its copies, frees its tensor memory and returns.
+// flag, frees its tensor memory and returns. (Copies that the fetching warp has in flight at that point are not waited for: their
+// barriers also expect producers that have left.)
 
 #include <algorithm>
 
